@@ -577,6 +577,10 @@ int spk_compact(spk_system *s, long long *freed) {
     s->xout_u.release();
     s->d_red_rows.release();
     s->d_red_off.release();
+    s->red_dense.release();
+    s->d_red_lv.release();
+    s->d_red_rr.release();
+    s->red_ring = 0;
     s->lean = 1;
     if (freed) *freed = before - spk_debug_scalar(s, "device_bytes");
     return SPK_OK;
@@ -635,6 +639,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
         b += s->T2.bytes() + s->IT2.bytes() + s->JT2.bytes() + s->S.bytes() + s->T.bytes() + s->IT.bytes();
         b += s->JT.bytes() + s->mapR.bytes() + s->dep.bytes() + s->mapRedX.bytes() + s->xbuf.bytes();
         b += s->xout_u.bytes() + s->d_tasks1.bytes() + s->d_tasks2.bytes() + s->d_red_rows.bytes();
+        b += s->red_dense.bytes() + s->d_red_lv.bytes() + s->d_red_rr.bytes();
         b += s->rdiag.bytes() + s->ell_val.bytes() + s->ell_col.bytes() + s->ell_ptr.bytes();
         b += s->ell_valf.bytes() + s->rdiagf.bytes() + s->diag.bytes() + s->rbuf.bytes() + s->dbuf.bytes() + s->work.bytes();
         b += s->stage_b.bytes() + s->stage_x.bytes();

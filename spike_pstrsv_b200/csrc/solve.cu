@@ -37,6 +37,7 @@
 #include <ctime>
 #include <mutex>
 
+#include "reduced.cuh"
 #include "spk_internal.cuh"
 
 namespace spk {
@@ -1210,107 +1211,6 @@ __device__ __forceinline__ double nanmax(double m, double v) { return (v > m || 
 
 // ---- batched solve support --------------------------------------------------------
 
-// Reduced solve on the kept rows for K right-hand sides stored in T with FP64
-// accumulation (same level structure as k_reduced_solve).  With FP32 storage and
-// an FP64 scratch `red` ([K][nred]), the reduced unknowns are gathered into it,
-// every level is solved and stored in FP64, and they are rounded to T once, on
-// the way back: the coupled boundary system stays FP64 throughout.
-template <int K>
-constexpr int red_threads() { return K >= 16 ? 512 : 1024; }  // K >= 16: registers for the K sums
-
-template <int K, typename T>
-__device__ __forceinline__ void reduced_body(const int *__restrict__ rows, const int *__restrict__ lvl_off, int nlvl,
-                                             const int *__restrict__ mapRedX, const int *__restrict__ IT,
-                                             const int *__restrict__ JT, const double *__restrict__ Tv,
-                                             T *__restrict__ xbuf, int n, double *__restrict__ red, int nred) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    if (red) {
-        for (long long e = threadIdx.x; e < (long long)K * nred; e += blockDim.x) {
-            const int k = (int)(e / nred), i = (int)(e % nred);
-            red[e] = (double)xbuf[(long long)k * n + mapRedX[i]];
-        }
-        __syncthreads();
-        for (int li = 0; li < nlvl; li++) {
-            for (int q = lvl_off[li] + warp; q < lvl_off[li + 1]; q += nwarps) {
-                const int kr = rows[q];
-                double sum[K];
-#pragma unroll
-                for (int k = 0; k < K; k++) sum[k] = 0.0;
-                for (int j = IT[kr] + lane; j < IT[kr + 1]; j += 32) {
-                    const int c = JT[j];
-#pragma unroll
-                    for (int k = 0; k < K; k++) sum[k] = fma(Tv[j], red[(long long)k * nred + c], sum[k]);
-                }
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-#pragma unroll
-                    for (int o = 16; o; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
-                }
-                if (lane == 0) {
-#pragma unroll
-                    for (int k = 0; k < K; k++) red[(long long)k * nred + kr] -= sum[k];
-                }
-            }
-            __syncthreads();
-        }
-        for (long long e = threadIdx.x; e < (long long)K * nred; e += blockDim.x) {
-            const int k = (int)(e / nred), i = (int)(e % nred);
-            xbuf[(long long)k * n + mapRedX[i]] = (T)red[e];
-        }
-        return;
-    }
-    for (int li = 0; li < nlvl; li++) {
-        for (int q = lvl_off[li] + warp; q < lvl_off[li + 1]; q += nwarps) {
-            const int kr = rows[q];
-            double sum[K];
-#pragma unroll
-            for (int k = 0; k < K; k++) sum[k] = 0.0;
-            for (int j = IT[kr] + lane; j < IT[kr + 1]; j += 32) {
-                const int c = mapRedX[JT[j]];
-#pragma unroll
-                for (int k = 0; k < K; k++) sum[k] = fma(Tv[j], (double)xbuf[(long long)k * n + c], sum[k]);
-            }
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-#pragma unroll
-                for (int o = 16; o; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
-            }
-            if (lane == 0) {
-                const long long r = mapRedX[kr];
-#pragma unroll
-                for (int k = 0; k < K; k++) xbuf[k * (long long)n + r] = (T)((double)xbuf[k * (long long)n + r] - sum[k]);
-            }
-        }
-        __syncthreads();
-    }
-}
-
-template <int K, typename T>
-__global__ void __launch_bounds__(red_threads<K>())
-k_reduced_solve_k(const int *__restrict__ rows, const int *__restrict__ lvl_off, int nlvl,
-                  const int *__restrict__ mapRedX, const int *__restrict__ IT, const int *__restrict__ JT,
-                  const double *__restrict__ Tv, T *__restrict__ xbuf, int n, double *__restrict__ red, int nred) {
-    reduced_body<K, T>(rows, lvl_off, nlvl, mapRedX, IT, JT, Tv, xbuf, n, red, nred);
-}
-
-// Reduced solves of many systems: block b takes the system of args[list[b]].
-struct RedArgs {
-    const int *rows, *lvl_off;
-    int nlvl;
-    const int *mapRedX, *IT, *JT;
-    const double *Tv;
-    void *xbuf;  // T
-    int n;
-    double *red;  // FP64 reduced unknowns of an FP32 batch ([K][nred]), or null
-    int nred;
-};
-
-template <int K, typename T>
-__global__ void __launch_bounds__(red_threads<K>()) k_reduced_multi(const RedArgs *__restrict__ args) {
-    const RedArgs A = args[blockIdx.x];
-    reduced_body<K, T>(A.rows, A.lvl_off, A.nlvl, A.mapRedX, A.IT, A.JT, A.Tv, (T *)A.xbuf, A.n, A.red, A.nred);
-}
-
 // R = B - A X in FP64 on the ELL copy (plus the diagonal), in the caller's order
 // (rev: caller row i is U row n-1-i).  One thread per row; a warp covers a tile.
 template <int K>
@@ -1658,29 +1558,6 @@ __global__ void k_reverse(int n, const double *__restrict__ src, double *__restr
         dst[i] = src[n - 1 - i];
 }
 
-// produceReducedY + __usol2 + updateX (ops.c:1152-1177, 1247-1262) in one CTA, on
-// the kept reduced rows: rows[] lists them level by level (a level is one
-// partition's dependents; its rows only reference later partitions), levels in
-// descending partition order, lvl_off[] delimiting the levels.  Dropped rows keep
-// y, so the gather/scatter only touches the kept rows and their columns.
-__global__ void __launch_bounds__(1024)
-k_reduced_solve(const int *__restrict__ rows, const int *__restrict__ lvl_off, int nlvl,
-                const int *__restrict__ mapRedX, const int *__restrict__ IT, const int *__restrict__ JT,
-                const double *__restrict__ T, double *__restrict__ xbuf) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int li = 0; li < nlvl; li++) {
-        for (int q = lvl_off[li] + warp; q < lvl_off[li + 1]; q += nwarps) {
-            const int k = rows[q];
-            double sum = 0.0;
-            for (int j = IT[k] + lane; j < IT[k + 1]; j += 32) sum = fma(T[j], xbuf[mapRedX[JT[j]]], sum);
-#pragma unroll
-            for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane == 0) xbuf[mapRedX[k]] -= sum;
-        }
-        __syncthreads();
-    }
-}
-
 // Absolute row sums of the dense spikes: first significant row per block
 // (everything above it is negligible) and the kept reduced rows.
 __global__ void k_first_significant(int nlist, const int *__restrict__ plist, const long long *__restrict__ startsS,
@@ -1912,18 +1789,22 @@ int solve_prepare(spk_system *s) {
         SPK_CUDA(cudaStreamSynchronize(s->stream));
         SPK_CUDA(cudaMemcpy(keep.data(), d_keep.p, sizeof(int) * s->rss, cudaMemcpyDeviceToHost));
     }
-    std::vector<int> rows, off{0};
+    std::vector<int> rows, off{0}, lvl_first;
     for (int t = P - 2; t >= 1; t--) {
         const int k0 = std::min(lvl[t], s->rss), k1 = std::min(lvl[t + 1], s->rss);
         const size_t before = rows.size();
         for (int k = k0; k < k1; k++)
             if (keep[k]) rows.push_back(k);
-        if (rows.size() > before) off.push_back((int)rows.size());
+        if (rows.size() > before) {
+            off.push_back((int)rows.size());
+            lvl_first.push_back(k0);
+        }
     }
     s->nlvl = (int)off.size() - 1;
     s->nkept = (int)rows.size();
     SPK_TRY(upload(s->d_red_rows, rows));
     SPK_TRY(upload(s->d_red_off, off));
+    SPK_TRY(reduced_prepare(s, rows, off, lvl_first));
 
     SPK_TRY(s->xbuf.alloc(s->n));
     if (s->uplo == 'L') SPK_TRY(s->xout_u.alloc(s->n));
@@ -2021,13 +1902,7 @@ int launch_tiles(spk_system *s, const double *rhs, long long ldb, double *xo, lo
         s->launches++;
     }
     if (prof) cudaEventRecord(s->ev[ring][1], st);
-    if (s->redNec && s->nkept) {
-        k_reduced_solve_k<K, T><<<1, red_threads<K>(), 0, st>>>(s->d_red_rows.p, s->d_red_off.p, s->nlvl, s->mapRedX.p,
-                                                     s->IT.p, s->JT.p, s->T.p, work, s->n,
-                                                     sizeof(T) == 4 ? s->red_scratch : nullptr, s->nRed);
-        SPK_CUDA(cudaGetLastError());
-        s->launches++;
-    }
+    if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, sizeof(T) == 4, K, work, st));
     if (prof) cudaEventRecord(s->ev[ring][2], st);
     A.tasks = s->d_tasks2.p;
     A.ntasks = s->ntasks2;
@@ -2080,13 +1955,7 @@ int launch_rhs(spk_system *s, int nk, const double *rhs, long long ldb, double *
         SPK_CUDA(cudaGetLastError());
         s->launches++;
     }
-    if (s->redNec && s->nkept) {
-        k_reduced_solve_k<32, T><<<1, red_threads<32>(), 0, st>>>(s->d_red_rows.p, s->d_red_off.p, s->nlvl, s->mapRedX.p,
-                                                      s->IT.p, s->JT.p, s->T.p, work, s->n,
-                                                      sizeof(T) == 4 ? s->red_scratch : nullptr, s->nRed);
-        SPK_CUDA(cudaGetLastError());
-        s->launches++;
-    }
+    if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, sizeof(T) == 4, nk, work, st));
     A.tasks = s->d_tasks2.p;
     A.ntasks = s->ntasks2;
     A.xfix = work;
@@ -2287,12 +2156,7 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
         }
         if (prof) cudaEventRecord(s->ev[ring][1], st);
         lap(1);
-        if (s->redNec && s->nkept) {
-            k_reduced_solve<<<1, 1024, 0, st>>>(s->d_red_rows.p, s->d_red_off.p, s->nlvl, s->mapRedX.p, s->IT.p,
-                                                s->JT.p, s->T.p, s->xbuf.p);
-            SPK_CUDA(cudaGetLastError());
-            s->launches++;
-        }
+        if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, 0, 1, s->xbuf.p, st));
         if (prof) cudaEventRecord(s->ev[ring][2], st);
         lap(2);
         A.tasks = TA.tasks = s->d_tasks2.p;
@@ -2657,8 +2521,8 @@ int clobber_rhs(spk_system *s, const double *x, double *b, cudaStream_t st) {
 // Every system's right-hand sides are split into width classes K in
 // {16, 8, 4, 2, 1} ("virtual systems": one system, K columns).  Per class, one
 // k_tile_multi launch runs the phase-1 tasks of all its virtual systems from a
-// flat work list (longest tasks first), one k_reduced_multi launch their
-// reduced solves (a block per virtual system), one k_tile_multi launch their
+// flat work list (longest tasks first), one launch per column block width their
+// reduced solves (reduced.cu; a cluster per system and column block), one k_tile_multi launch their
 // phase 3+4 tasks; FP32 + refinement adds k_residual_multi and k_axpy_multi
 // over flat row-block lists.  The whole sequence is captured once into a CUDA
 // graph and replayed by spk_group_solve.
@@ -2685,9 +2549,9 @@ struct GroupClass {
     int K = 0;
     DBuf<TileArgs> a1, a4, c1, c4;  // solve and correction-solve arguments (phase 1, phase 3+4)
     DBuf<int2> w1, w4, vw;
-    DBuf<RedArgs> red, cred;
+    RedPlan red;  // the class's reduced solves
     DBuf<VecArgs> va;
-    int n1 = 0, n4 = 0, nred = 0, nvw = 0;
+    int n1 = 0, n4 = 0, nvw = 0;
     std::vector<int> vs;  // virtual systems of the class
 };
 
@@ -2705,6 +2569,7 @@ struct spk_group {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;
+    int rc = SPK_OK;  // first failed launch of the capture
 };
 
 namespace spk {
@@ -2751,7 +2616,7 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
                 const std::vector<std::vector<SegTask>> &t4) {
     const bool fp32 = g->mode == 1;
     std::vector<TileArgs> a1, a4, c1, c4;
-    std::vector<RedArgs> red, cred;
+    std::vector<RedMember> red;
     std::vector<VecArgs> va;
     std::vector<std::pair<long long, int2>> w1, w4;
     std::vector<int2> vw;
@@ -2773,12 +2638,7 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
             const SegTask &q = t4[v.sys][t];
             w4.push_back({(long long)(q.hi - q.lo) + (q.tail - q.hi), make_int2((int)i, t)});
         }
-        if (s->redNec && s->nkept) {
-            RedArgs r{s->d_red_rows.p, s->d_red_off.p, s->nlvl, s->mapRedX.p, s->IT.p, s->JT.p, s->T.p, v.work,
-                      s->n, fp32 ? v.red : nullptr, s->nRed};
-            red.push_back(r);
-            cred.push_back(r);
-        }
+        if (s->redNec && s->nkept) red.push_back(RedMember{s, v.work, v.red});
         VecArgs a{};
         a.n = s->n;
         a.rev = s->uplo == 'L';
@@ -2813,10 +2673,7 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
     SPK_TRY(upload_vec(c.w4, s4));
     c.n1 = (int)s1.size();
     c.n4 = (int)s4.size();
-    // reduced solves: one argument block per virtual system that has a reduced system
-    SPK_TRY(upload_vec(c.red, red));
-    SPK_TRY(upload_vec(c.cred, cred));
-    c.nred = (int)red.size();
+    SPK_TRY(red_plan_build(c.red, red, c.K, fp32));
     SPK_TRY(upload_vec(c.va, va));
     SPK_TRY(upload_vec(c.vw, vw));
     c.nvw = (int)vw.size();
@@ -2831,10 +2688,7 @@ void enqueue_solve(spk_group *g, GroupClass &c, bool correction, cudaStream_t st
         k_tile_multi<false, K, T, T><<<c.n1, 32, 0, st>>>(p1, c.w1.p);
         g->kernels++;
     }
-    if (c.nred) {
-        k_reduced_multi<K, T><<<c.nred, red_threads<K>(), 0, st>>>(c.red.p);
-        g->kernels++;
-    }
+    if (const int rc = red_plan_launch(c.red, st, &g->kernels); rc != SPK_OK) g->rc = rc;
     if (c.n4) {
         k_tile_multi<true, K, T, double><<<c.n4, 32, 0, st>>>(p4, c.w4.p);
         g->kernels++;
@@ -2990,6 +2844,10 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
     }
     enqueue_all(g, st);
     cudaError_t e = cudaStreamEndCapture(st, &g->graph);
+    if (g->rc != SPK_OK) {
+        (void)cudaGetLastError();
+        return fail(g->rc);
+    }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();

@@ -215,6 +215,13 @@ struct spk_system {
     int pipe_K = 0, pipe_nograph = 0;
     spk::DBuf<int> d_red_rows, d_red_off, d_err;  // kept reduced rows by level; device error flag
     int nlvl = 0, nkept = 0;
+    // reduced solve on a cluster (reduced.cu): levels (8 ints each), kept rows (reduced
+    // unknown, U row, first and last entry), dense coefficients where those are few
+    spk::DBuf<int> d_red_lv;
+    spk::DBuf<int4> d_red_rr;
+    spk::DBuf<double> red_dense;
+    int red_ring = 0;   // unknowns a level spans (0: the one-CTA solve on the CSR copy)
+    int red_ctas = 1;   // CTAs per cluster
     int dbg_fail_waits = 0;  // test hook: solve kernels report a failed wait at entry (spk_debug_set)
     int lean = 0;  // spk_compact: only what the chain solves read is kept (partition paths refused)
     double *red_scratch = nullptr;  // FP64 reduced unknowns of the FP32 batched solve in flight
@@ -241,6 +248,9 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
 int solve_batch_static(spk_system *s, int nrhs, const double *B, long long ldb, double *X, long long ldx,
                        cudaStream_t st);
 int solve_prepare(spk_system *s);
+int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vector<int> &off,
+                    const std::vector<int> &lvl_first);
+int reduced_solve(spk_system *s, int fp32, int ncols, void *work, cudaStream_t st);
 int residual_prepare(spk_system *s);
 int chain_prepare(spk_system *s);
 int chain_tune(spk_system *s, const char *name, long long v);
