@@ -581,6 +581,7 @@ int spk_compact(spk_system *s, long long *freed) {
     s->d_red_lv.release();
     s->d_red_rr.release();
     s->red_ring = 0;
+    s->d_copies.release();
     s->lean = 1;
     if (freed) *freed = before - spk_debug_scalar(s, "device_bytes");
     return SPK_OK;
@@ -607,6 +608,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
         return (s->redNec && s->ntasks1 ? 1 : 0) + (s->redNec && s->nkept ? 1 : 0) + 1;
     }
     if (!strcmp(name, "chain")) return s->chain_ok;
+    if (!strcmp(name, "sweep")) return s->sw_ok;
     if (!strcmp(name, "lean")) return s->lean;
     if (!strcmp(name, "device_check")) return chain_device_check();  // checked builds only
     if (!strcmp(name, "chains")) return s->ch_count;
@@ -639,6 +641,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
         b += s->T2.bytes() + s->IT2.bytes() + s->JT2.bytes() + s->S.bytes() + s->T.bytes() + s->IT.bytes();
         b += s->JT.bytes() + s->mapR.bytes() + s->dep.bytes() + s->mapRedX.bytes() + s->xbuf.bytes();
         b += s->xout_u.bytes() + s->d_tasks1.bytes() + s->d_tasks2.bytes() + s->d_red_rows.bytes();
+        b += s->sw_rec.bytes() + s->sw_hdr.bytes() + s->d_copies.bytes();
         b += s->red_dense.bytes() + s->d_red_lv.bytes() + s->d_red_rr.bytes();
         b += s->rdiag.bytes() + s->ell_val.bytes() + s->ell_col.bytes() + s->ell_ptr.bytes();
         b += s->ell_valf.bytes() + s->rdiagf.bytes() + s->diag.bytes() + s->rbuf.bytes() + s->dbuf.bytes() + s->work.bytes();

@@ -48,6 +48,7 @@
 #include <vector>
 
 #include "spk_internal.cuh"
+#include "sweep.cuh"
 
 namespace spk {
 
@@ -460,8 +461,21 @@ size_t chain_smem_bytes(const spk_system *s) {
 }
 
 template <bool PRE>
-int launch_chain(spk_system *s, const ChainTask *tasks, int ntasks, const double *b, double *x, cudaStream_t st) {
+int launch_chain(spk_system *s, const ChainTask *tasks, int ntasks, const double *b, double *x, cudaStream_t st,
+                 bool dependent = false) {
     if (ntasks <= 0) return SPK_OK;
+    if (s->sw_ok) {
+        SweepArgs W = sweep_args(s);
+        W.tasks = tasks;
+        W.ntasks = ntasks;
+        W.b = b;
+        W.x = x;
+        W.pre = PRE ? x : nullptr;
+        W.rev_b = W.rev_x = W.rev_pre = s->uplo == 'L';
+        SPK_TRY(sweep_launch(s, W, dependent, st));
+        s->launches++;
+        return SPK_OK;
+    }
     ChainArgs A;
     A.tasks = tasks;
     A.val = s->ch_val.p;
@@ -1086,8 +1100,10 @@ int chain_prepare(spk_system *s) {
     SPK_CUDA(cudaGetDevice(&dev));
     SPK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     SPK_TRY(chain_occupancy(s, &occ));
-    // (seven per SM at most: with more, phase 1 gains nothing and phase 4 grows)
-    long long len = 32ll * ((n / (sms * (long long)std::min(std::max(occ, 1), 7)) + 31) / 32);
+    // (on 16-row records six per SM at most, on 32-row tiles seven: with more, phase 1
+    // gains nothing and phase 4 grows.  Records, full-size banded rows: 290 / 231 / 211 /
+    // 194 us with 3 / 4 / 5 / 6)
+    long long len = 32ll * ((n / (sms * (long long)std::min(std::max(occ, 1), s->sw_ok ? 6 : 7)) + 31) / 32);
     len = std::max<long long>(len, 1024);
     if (const char *e = getenv("SPK_CHAIN_ROWS")) len = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     SPK_TRY(build_plan(s, len, reach, nullptr));
@@ -1165,6 +1181,7 @@ int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra) {
 
 // Resident blocks per SM of the phase-1 solve kernel (its shared memory bounds it).
 int chain_occupancy(spk_system *s, int *occ) {
+    if (s->sw_ok) return sweep_occupancy(s, occ);
     const size_t smem = chain_smem_bytes(s);
     auto q = [&](auto kern) -> int {
         SPK_TRY(allow_smem(kern));
@@ -1406,7 +1423,7 @@ int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool
         cudaEventRecord(s->ev[ring][1], st);
         cudaEventRecord(s->ev[ring][2], st);
     }
-    SPK_TRY(launch_chain<true>(s, s->d_ctasks4.p, s->nctasks4, b, x, st));
+    SPK_TRY(launch_chain<true>(s, s->d_ctasks4.p, s->nctasks4, b, x, st, !prof));
     return SPK_OK;
 }
 

@@ -39,6 +39,7 @@
 
 #include "reduced.cuh"
 #include "spk_internal.cuh"
+#include "sweep.cuh"
 
 namespace spk {
 
@@ -1720,7 +1721,7 @@ int build_seg_tasks(spk_system *s, const std::vector<int> &first, const std::vec
     s->rows_phase4 = rows2;
     SPK_TRY(upload(s->d_tasks1, t1));
     SPK_TRY(upload(s->d_tasks2, t2));
-    return SPK_OK;
+    return sweep_copies(s, t2);
 }
 
 int solve_prepare(spk_system *s) {
@@ -1854,6 +1855,7 @@ int solve_prepare(spk_system *s) {
     SPK_TRY(s->d_err.alloc(1));
     SPK_CUDA(cudaMemset(s->d_err.p, 0, sizeof(int)));
     mark(3);  // 1/diagonal, sliced ELL
+    SPK_TRY(sweep_prepare(s));
     SPK_TRY(chain_prepare(s));
     if (!s->chain_ok) SPK_TRY(partition_ensure(s));
     mark(4);  // chain layout, spikes and plans (or the internal spikes without chains)
@@ -1873,12 +1875,47 @@ int partition_ensure(spk_system *s) {
 
 namespace {
 
+// Phase 1 (into work, U order) and phase 3+4 of one right-hand side on 16-row records.
+int sweep_phase(spk_system *s, bool phase4, const double *rhs, double *xo, double *work, bool dependent,
+                cudaStream_t st) {
+    SweepArgs A = sweep_args(s);
+    A.b = rhs;
+    A.rev_b = s->uplo == 'L';
+    if (phase4) {
+        A.tasks = s->d_tasks2.p;
+        A.ntasks = s->ntasks2;
+        A.copies = s->d_copies.p;
+        A.ncopies = s->ncopies;
+        A.x = xo;
+        A.rev_x = s->uplo == 'L';
+        A.pre = work;
+    } else {
+        A.tasks = s->d_tasks1.p;
+        A.ntasks = s->ntasks1;
+        A.x = work;
+    }
+    A.seg = 1;
+    SPK_TRY(sweep_launch(s, A, dependent, st));
+    s->launches++;
+    return SPK_OK;
+}
+
+int sweep_tiles(spk_system *s, const double *rhs, double *xo, double *work, cudaStream_t st, bool prof, int ring) {
+    if (s->redNec && s->ntasks1) SPK_TRY(sweep_phase(s, false, rhs, nullptr, work, false, st));
+    if (prof) cudaEventRecord(s->ev[ring][1], st);
+    if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, 0, 1, work, st));
+    if (prof) cudaEventRecord(s->ev[ring][2], st);
+    return sweep_phase(s, true, rhs, xo, work, !prof && s->redNec && s->ntasks1, st);
+}
+
 // One Spike solve of K right-hand sides with the tile solver: phase 1 into the
 // U-order work buffer (T, leading dimension n), the kept reduced rows, phase 3+4
 // into xo (FP64, caller order).
 template <int K, typename T>
 int launch_tiles(spk_system *s, const double *rhs, long long ldb, double *xo, long long ldx, T *work,
                  cudaStream_t st, bool prof, int ring) {
+    if constexpr (K == 1 && sizeof(T) == 8)
+        if (s->sw_ok) return sweep_tiles(s, rhs, xo, work, st, prof, ring);
     TileArgs A{};
     A.ell_val = sizeof(T) == 8 ? (const void *)s->ell_val.p : (const void *)s->ell_valf.p;
     A.ell_col = s->ell_col.p;
@@ -2115,7 +2152,7 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
     }
     if (s->chain_ok && (!ph || s->lean)) {  // a compacted system has no other path (no phase times)
         SPK_TRY(chain_solve(s, b, x, st, prof, ring));
-    } else if (s->ell_ok && !ph) {
+    } else if ((s->ell_ok || s->sw_ok) && !ph) {
         SPK_TRY((launch_tiles<1, double>(s, b, s->n, x, s->n, s->xbuf.p, st, prof, ring)));
     } else {
         // CSR segment solver (or the timed legacy path, which times the phases)
@@ -2149,10 +2186,14 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
             TA.xout = s->xbuf.p;
             TA.ldx = s->n;
             A.rev_out = TA.rev_out = 0;
-            if (s->ell_ok) k_tile_solve<false, 1, double, double><<<s->ntasks1, 32, 0, st>>>(TA);
-            else k_segment_solve<false><<<s->ntasks1, 32, 0, st>>>(A);
-            SPK_CUDA(cudaGetLastError());
-            s->launches++;
+            if (s->sw_ok) {
+                SPK_TRY(sweep_phase(s, false, b, nullptr, s->xbuf.p, false, st));
+            } else {
+                if (s->ell_ok) k_tile_solve<false, 1, double, double><<<s->ntasks1, 32, 0, st>>>(TA);
+                else k_segment_solve<false><<<s->ntasks1, 32, 0, st>>>(A);
+                SPK_CUDA(cudaGetLastError());
+                s->launches++;
+            }
         }
         if (prof) cudaEventRecord(s->ev[ring][1], st);
         lap(1);
@@ -2167,10 +2208,14 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
         TA.xout = x;
         TA.ldx = s->n;
         A.rev_out = TA.rev_out = s->uplo == 'L';
-        if (s->ell_ok) k_tile_solve<true, 1, double, double><<<s->ntasks2, 32, 0, st>>>(TA);
-        else k_segment_solve<true><<<s->ntasks2, 32, 0, st>>>(A);
-        SPK_CUDA(cudaGetLastError());
-        s->launches++;
+        if (s->sw_ok) {
+            SPK_TRY(sweep_phase(s, true, b, x, s->xbuf.p, false, st));
+        } else {
+            if (s->ell_ok) k_tile_solve<true, 1, double, double><<<s->ntasks2, 32, 0, st>>>(TA);
+            else k_segment_solve<true><<<s->ntasks2, 32, 0, st>>>(A);
+            SPK_CUDA(cudaGetLastError());
+            s->launches++;
+        }
     }
     if (prof) {
         cudaEventRecord(s->ev[ring][3], st);

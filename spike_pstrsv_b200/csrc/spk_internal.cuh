@@ -192,6 +192,12 @@ struct spk_system {
     spk::ChainPlan cp_batch;  // the batched kernel's own chains (longer; built at preprocessing)
     spk::ChainPlan cp_host;   // the host-array pipeline's chains (shorter; built on first use)
     int batch_path = -1;      // spk_tune "batch_path": 1 chain kernels, 0 partition kernels, -1 automatic
+    // 16-row records of U for the one-right-hand-side solves (sweep.cu)
+    int sw_ok = 0, sw_win = 0, sw_reach = 0, sw_wide = 0, sw_slots = 0, sw_stage = 0;
+    spk::DBuf<unsigned char> sw_rec;
+    spk::DBuf<int2> sw_hdr;
+    spk::DBuf<int2> d_copies;  // phase 3+4: row ranges that keep their phase-1 values
+    int ncopies = 0;
     // wall milliseconds of the last preprocessing: the reference's steps, first
     // significant spike rows + internal spikes, reduced levels + buffers, the
     // sliced-ELL layout, the chain layout and plans (spk_debug_scalar "prep_us_*")
