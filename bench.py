@@ -473,8 +473,11 @@ def run_ours(args):
     ph = kernel_time_per_solve(S, db, dx, sp, dev, args.steps)
     chain = S.scalar("chain") == 1
     if chain:
-        rows1, rows4 = S.scalar("chain_rows_phase1"), S.scalar("chain_rows_phase4")
-        kernel = "k_chain_solve (phase 1 chain-local sweep + phase 4 re-solve of the coupled rows), 2 launches per solve"
+        one = S.scalar("launches_per_solve") == 1
+        rows1 = S.scalar("chain_solve_rows") if one else S.scalar("chain_rows_phase1")
+        rows4 = 0 if one else S.scalar("chain_rows_phase4")
+        kernel = ("k_sweep (tasks of rows, each started where its own rows no longer feel the start), 1 launch per solve"
+                  if one else "phase 1 chain-local sweep + phase 4 re-solve of the coupled rows, 2 launches per solve")
     else:
         rows1, rows4 = S.scalar("rows_phase1"), S.scalar("rows_phase4")
         kernel = "k_tile_solve (phase 1 D1 sweep + phase 3/4 coupled D2 sweep), 2 launches per solve"

@@ -308,8 +308,9 @@ int spk_compact(spk_system *s, long long *freed);
 /* Tuning knobs of a system solved by chains (no reference counterpart; the
  * reference's only knob is nthreads).  spk_debug_scalar(s, name) reads them back.
  *   "rows":       rows per chain task of the one-right-hand-side solve (rounded
- *                 up to whole 32-row tiles, doubled at most three times until
- *                 every chain keeps its first rows final; SPK_ERR_ARG if none)
+ *                 up to whole 32-row tiles; in the two-phase form doubled at
+ *                 most three times until every chain keeps its first rows
+ *                 final; SPK_ERR_ARG if none)
  *   "batch_rows": the same for the batched solve's own chains
  *   "stages":     2 or 3 tiles staged ahead by the one-right-hand-side kernel
  *   "batch_path": 1 batched solves on the chain kernels, 0 on the partition

@@ -604,7 +604,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
     if (!strcmp(name, "ell")) return s->ell_ok;
     if (!strcmp(name, "ell_entries")) return s->ell_entries;
     if (!strcmp(name, "launches_per_solve")) {
-        if (s->chain_ok) return (s->nctasks1 ? 1 : 0) + (s->nctasks4 ? 1 : 0);
+        if (s->chain_ok || s->ov.len) return s->ov.len ? 1 : (s->nctasks1 ? 1 : 0) + (s->nctasks4 ? 1 : 0);
         return (s->redNec && s->ntasks1 ? 1 : 0) + (s->redNec && s->nkept ? 1 : 0) + 1;
     }
     if (!strcmp(name, "chain")) return s->chain_ok;
@@ -613,6 +613,11 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
     if (!strcmp(name, "device_check")) return chain_device_check();  // checked builds only
     if (!strcmp(name, "chains")) return s->ch_count;
     if (!strcmp(name, "chain_rows")) return s->ch_len;
+    if (!strcmp(name, "chain_solve_rows")) {  // rows that one solve walks
+        long long r = s->ov.len ? 0 : s->ch_rows1 + s->ch_rows4;
+        for (const ChainTask &t : s->ov.h1) r += t.hi - t.lo;
+        return r;
+    }
     if (!strcmp(name, "chain_width")) return s->ch_width;
     if (!strcmp(name, "chain_reach")) return s->ch_reach;
     if (!strcmp(name, "chain_rows_phase1")) return s->ch_rows1;
@@ -626,11 +631,11 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
             if (!strcmp(name + 8, parts[i])) return (long long)(s->prep_ms[i] * 1e3);
     }
     // spk_tune's knobs under their own names
-    if (!strcmp(name, "rows")) return s->ch_len;
+    if (!strcmp(name, "rows")) return s->ov.len ? s->ov.len : s->ch_len;
     if (!strcmp(name, "batch_rows")) return s->cp_batch.len ? s->cp_batch.len : s->ch_len;
     if (!strcmp(name, "stages")) return s->ch_stages;
     if (!strcmp(name, "batch_path")) return s->batch_path;
-    if (!strcmp(name, "chain_host_rows")) return s->cp_host.len ? s->cp_host.len : s->ch_len;
+    if (!strcmp(name, "chain_host_rows")) return s->ov_host.len ? s->ov_host.len : s->ov.len ? s->ov.len : s->cp_host.len ? s->cp_host.len : s->ch_len;
     if (!strcmp(name, "chain_bytes")) return (long long)(s->ch_val.bytes() + s->ch_off.bytes() + s->ch_ptr.bytes());
     if (!strcmp(name, "rows_phase4")) return s->rows_phase4;
     if (!strcmp(name, "kept_reduced_rows")) return s->nkept;
@@ -647,7 +652,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
         b += s->ell_valf.bytes() + s->rdiagf.bytes() + s->diag.bytes() + s->rbuf.bytes() + s->dbuf.bytes() + s->work.bytes();
         b += s->stage_b.bytes() + s->stage_x.bytes();
         b += s->ch_val.bytes() + s->ch_valb.bytes() + s->ch_valbf.bytes() + s->ch_near.bytes() + s->ch_nearf.bytes() + s->ch_off.bytes() + s->ch_ptr.bytes() + s->d_ctasks1.bytes() +
-             s->d_ctasks4.bytes();
+             s->d_ctasks4.bytes() + s->ov.d1.bytes() + s->ov_host.d1.bytes();
         return b;
     }
     return -1;

@@ -22,7 +22,19 @@
 // values.  Preprocessing doubles the chain length until that holds, and falls
 // back to the partition-based solve otherwise.
 //
-// Kernel.  One warp per task, lane = row of a 32-row tile, tiles bottom-up.  The
+// One launch.  Where the system has 16-row records (sweep.cu), the one-right-hand-side
+// solve needs no second phase: a task for rows [a, q) starts `ov_warm` rows below, at
+// q + ov_warm, with zero coupling there, and stores only its own rows.  What the start
+// leaves out reaches rows [q, q + reach) as a spike of at most tau (the spike of
+// [q, q + ov_warm) is computed exactly and checked for every q), so the window holds
+// the same values there as phase 4 would read.  The rows walked are those of both
+// phases plus `reach` a task, but the tasks need no other task's rows: their number
+// is free, down to 32 rows, and the walk's length is a + ov_warm instead of at least
+// twice the decay length.  262,147 rows, transpose: 80 -> 48 us; 5,003 rows: 47 -> 27 us.
+// spk_chain_phase keeps the two phases (a shard's rows end where another GPU's start).
+//
+// Kernel (systems without records, and the phases' layout).  One warp per task, lane = row of
+// a 32-row tile, tiles bottom-up.  The
 // matrix is stored for this solver as a sliced ELL of ROW-SCALED off-diagonals
 // a(r,c)/a(r,r) (so x_r = b_r/a(r,r) - sum v'(r,c) x_c) with 8-bit column
 // offsets c - r, per tile slot-pair-major (values: one 16-byte copy per lane per
@@ -1010,7 +1022,7 @@ int chain_batch_values(spk_system *s, int fp32) {
     return SPK_OK;
 }
 
-void chain_release(spk_system *s) {
+void chain_release(spk_system *s, bool keep_overlap = false) {
     s->chain_ok = 0;
     s->batch_path = -1;
     s->ch_val.release();
@@ -1024,6 +1036,11 @@ void chain_release(spk_system *s) {
     s->d_ctasks4.release();
     s->cp_batch.release();
     s->cp_host.release();
+    if (!keep_overlap) {
+        s->ov.release();
+        s->ov_host.release();
+        s->ov_warm = 0;
+    }
     s->host_plan_tried = 0;
     if (s->pipe_exec) cudaGraphExecDestroy(s->pipe_exec);
     s->pipe_exec = nullptr;
@@ -1043,6 +1060,9 @@ void chain_release(spk_system *s) {
 int chain_occupancy(spk_system *s, int *occ);
 int chain_rhs_occupancy(spk_system *s, int *occ);
 int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra);
+long long overlap_rows(spk_system *s, int sms, int occ);
+long long overlap_warm(const spk_system *s);
+int build_overlap(spk_system *s, long long len, ChainPlan &out);
 
 // Build the chain layout, the chains' spikes and the two task lists; leaves
 // chain_ok = 0 (the partition-based solve) when truncation is off, the layout
@@ -1107,7 +1127,13 @@ int chain_prepare(spk_system *s) {
     len = std::max<long long>(len, 1024);
     if (const char *e = getenv("SPK_CHAIN_ROWS")) len = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     SPK_TRY(build_plan(s, len, reach, nullptr));
-    if (!s->chain_ok) return SPK_OK;
+    if (!s->chain_ok) {
+        // too few rows for chains that keep their first rows, but the spikes may decay
+        // all the same: the one-launch solve needs no more
+        if (s->sw_ok && s->ov_warm && s->ov_warm < n) SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
+        chain_release(s, true);
+        return SPK_OK;
+    }
     // the batched kernel keeps fewer tasks resident (a wider window): its own
     // chains, as many as it keeps resident
     int occb = 4;
@@ -1116,14 +1142,74 @@ int chain_prepare(spk_system *s) {
     lenb = std::max<long long>(lenb, s->ch_len);
     if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) lenb = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     if (lenb > s->ch_len) SPK_TRY(build_plan(s, lenb, reach, &s->cp_batch));
+    if (s->sw_ok) SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
+    return SPK_OK;
+}
+
+// Rows per task of the one-launch solve.  With w tasks an SM a task walks n / (sms w) +
+// ov_warm rows: more tasks shorten the walk, but slow each other down and together
+// walk more rows, until the records saturate HBM.  Measured, w = 1 .. 6: 262,147 banded
+// rows 78 / 57 / 57 / 53 / 55 / 55 us, 4,194,304 rows 706 / 371 / 295 / 232 / 213 / 189 us (the
+// transpose, with longer records, 235 us from w = 4 on), 65,536 rows 46 / 41 / 44 / 43 / 47 us;
+// the model is within 6 % of those: 0.27 us and 0.012 us a slot per tile, 6 % more for
+// each further task, 6.5 TB/s.
+long long overlap_rows(spk_system *s, int sms, int occ) {
+    if (const char *e = getenv("SPK_CHAIN_ROWS")) return std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
+    const long long n = s->n, warm = overlap_warm(s);
+    const double tile_ns = 270 + 12.0 * s->sw_slots, row_bytes = (double)s->sw_rec.n / n + 16;
+    long long best = 0;
+    double best_t = 0;
+    for (int w = 1; w <= std::min(std::max(occ, 1), 6); w++) {
+        const long long len = std::max(32ll, 32ll * ((n / (sms * (long long)w) + 31) / 32));
+        const double walk = std::min(len + warm, n) / 16.0 * tile_ns * (1 + 0.06 * (w - 1));
+        const double t = std::max(walk, n * (1.0 + (double)warm / len) * row_bytes / 6500);
+        if (!best || t < best_t) best = len, best_t = t;
+    }
+    return best;
+}
+
+// The decay length of the plan's spikes, and the rows that a task's first row may read.
+long long overlap_warm(const spk_system *s) {
+    if (s->ov_warm) return s->ov_warm;
+    long long redo = 0;
+    for (const ChainTask &t : s->h_ctasks1) redo = std::max<long long>(redo, t.hi - t.st_hi);
+    return 32ll * ((redo + s->ch_reach + 31) / 32);
+}
+
+// Tasks of `len` rows for the one-launch solve: the start below each task is raised until
+// the spike of the rows walked before the task's own is negligible in the first `reach`
+// of them, for every task; left empty (two phases) if it does not become so.
+int build_overlap(spk_system *s, long long len, ChainPlan &out) {
+    const int n = s->n;
+    out.release();
+    long long warm = overlap_warm(s);
+    for (int tries = 0; tries < 6; tries++, warm += 32 * (warm / 128 + 1)) {
+        std::vector<int2> segs;
+        for (long long q = len; q + warm < n; q += len) segs.push_back(make_int2((int)q, (int)(q + warm)));
+        bool ok = true;
+        if (!segs.empty()) {
+            std::vector<int> first;
+            SPK_TRY(spike_firsts(s, segs, first));
+            for (size_t c = 0; c < segs.size() && ok; c++) ok = first[c] >= segs[c].x + s->ch_reach;
+        }
+        if (!ok) continue;
+        for (long long a = 0; a < n; a += len) {
+            const long long q = std::min<long long>(a + len, n);
+            out.h1.push_back(ChainTask{(int)a, (int)std::min<long long>(q + warm, n), (int)a, (int)q});
+        }
+        SPK_TRY(upload_vec(out.d1, out.h1));
+        out.len = (int)len;
+        s->ov_warm = (int)warm;
+        return SPK_OK;
+    }
     return SPK_OK;
 }
 
 // Chains of `len` rows (doubled up to three times until every chain keeps its
 // first `reach` rows, never fewer than 8 chains): their spikes, the two task
 // lists (row order: the pipelined and sharded solves launch them by row range).
-// extra == nullptr: the plain solve's plan (sets chain_ok, or releases everything
-// when no length is valid); else a second plan (left unbuilt, so that the plain
+// extra == nullptr: the plain solve's plan (sets chain_ok, or leaves ov_warm when no
+// length is valid but the spikes decay); else a second plan (left unbuilt, so that the plain
 // plan's tasks are used, when no length short of the plain one is valid).
 int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra) {
     const int n = s->n;
@@ -1138,7 +1224,15 @@ int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra) {
         bool ok = true;
         for (size_t c = 1; c < chains.size() && ok; c++)
             ok = first[c] >= std::min(chains[c].x + reach, chains[c].y);
-        if (!ok) continue;
+        if (!ok) {
+            // the decay length, where every chain holds it (the top chain's spike is never cut off)
+            int redo = 0;
+            for (size_t c = 1; c < chains.size(); c++)
+                redo = first[c] > chains[c].x ? std::max(redo, chains[c].y - first[c]) : n;
+            if (!extra) s->ov_warm = redo + reach < n ? 32 * ((redo + reach + 31) / 32) : 0;
+            continue;
+        }
+        if (!extra) s->ov_warm = 0;
         std::vector<ChainTask> t1, t4;
         long long rows1 = 0, rows4 = 0;
         for (size_t c = 0; c < chains.size(); c++) {
@@ -1175,7 +1269,6 @@ int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra) {
         extra->release();  // the plain solve's tasks are used
         return SPK_OK;
     }
-    chain_release(s);
     return SPK_OK;
 }
 
@@ -1234,9 +1327,14 @@ int chain_solve_host(spk_system *s, const double *b, double *x, double *db, doub
         s->host_plan_tried = 1;
         long long len = 2048;
         if (const char *e = getenv("SPK_PIPELINE_ROWS")) len = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
-        if (len < s->ch_len) SPK_TRY(build_plan(s, len, s->ch_reach, &s->cp_host));
+        if (s->ov.len) {
+            if (len < s->ov.len) SPK_TRY(build_overlap(s, len, s->ov_host));
+        } else if (len < s->ch_len) {
+            SPK_TRY(build_plan(s, len, s->ch_reach, &s->cp_host));
+        }
     }
-    const int nch = (int)(s->cp_host.len > 0 ? s->cp_host.h1.size() : s->h_ctasks1.size());
+    const int nch = (int)(s->ov_host.len ? s->ov_host.h1.size() : s->ov.len ? s->ov.h1.size()
+                          : s->cp_host.len > 0 ? s->cp_host.h1.size() : s->h_ctasks1.size());
     int K = 16;
     if (const char *e = getenv("SPK_PIPELINE_CHUNKS")) K = std::max(1, atoi(e));
     K = std::min(K, std::max(nch, 1));
@@ -1308,12 +1406,15 @@ int chain_solve_host(spk_system *s, const double *b, double *x, double *db, doub
 // system's stream (nothing here synchronizes: it may be captured).
 int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double *dx, int K) {
     const ChainPlan &hp = s->cp_host;
-    const bool own = hp.len > 0;
-    const std::vector<ChainTask> &T1 = own ? hp.h1 : s->h_ctasks1, &T4 = own ? hp.h4 : s->h_ctasks4;
-    const ChainTask *D1 = own ? hp.d1.p : s->d_ctasks1.p, *D4 = own ? hp.d4.p : s->d_ctasks4.p;
+    const bool own = hp.len > 0, one = s->ov.len > 0;  // one: no phase 4
+    const ChainPlan &op = s->ov_host.len ? s->ov_host : s->ov;
+    const std::vector<ChainTask> &T1 = one ? op.h1 : own ? hp.h1 : s->h_ctasks1, &T4 = one ? op.h4 : own ? hp.h4 : s->h_ctasks4;
+    const ChainTask *D1 = one ? op.d1.p : own ? hp.d1.p : s->d_ctasks1.p, *D4 = own ? hp.d4.p : s->d_ctasks4.p;
     const int n = s->n, nch = (int)T1.size(), n4 = (int)T4.size();
     cudaEvent_t *ev_in = s->pipe_ev.data(), *ev_p1 = ev_in + K, *ev_done = ev_in + 2 * K, *ev_start = ev_in + 3 * K;
     const bool rev = s->uplo == 'L';
+    // the end of a task's own rows (its walk may start further below)
+    auto own_end = [&](const std::vector<ChainTask> &T, int c) { return c + 1 < (int)T.size() ? T[c + 1].lo : n; };
     // chunk k: chains [c0(k), c0(k+1)), U rows [A(k), Q(k)), phase-4 tasks [t0(k), t0(k+1))
     std::vector<int> c0(K + 1), t0(K + 1, 0);
     for (int k = 0; k <= K; k++) c0[k] = (int)((long long)nch * k / K);
@@ -1321,13 +1422,13 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
         int t = 0;
         for (int k = 0; k < K; k++) {
             t0[k] = t;
-            const int qend = T1[c0[k + 1] - 1].hi;
+            const int qend = own_end(T1, c0[k + 1] - 1);
             while (t < n4 && T4[t].hi <= qend) t++;
         }
         t0[K] = n4;
     }
     auto lo_rows = [&](int k, int &lo, int &cnt) {
-        const int A = T1[c0[k]].lo, Q = T1[c0[k + 1] - 1].hi;
+        const int A = T1[c0[k]].lo, Q = own_end(T1, c0[k + 1] - 1);
         lo = rev ? n - Q : A;
         cnt = Q - A;
     };
@@ -1345,7 +1446,19 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
     // rows of chunk k) right behind it on the same stream: streams share the
     // device's hardware queues, and a launch queued behind one it does not
     // depend on would wait for it
-    for (int k = 0; k <= K; k++) {
+    // (one launch: chunk k's walks start in a later chunk's rows; its x leaves when it is done)
+    for (int k = 0; one && k < K; k++) {
+        cudaStream_t q = s->pipe_st[k];
+        int last = k, lo, cnt;
+        while (last + 1 < K && own_end(T1, c0[last + 1] - 1) < T1[c0[k + 1] - 1].hi) last++;
+        SPK_CUDA(cudaStreamWaitEvent(q, ev_in[last], 0));
+        SPK_TRY(launch_chain<false>(s, D1 + c0[k], c0[k + 1] - c0[k], db, dx, q));
+        SPK_CUDA(cudaEventRecord(ev_done[k], q));
+        lo_rows(k, lo, cnt);
+        SPK_CUDA(cudaStreamWaitEvent(s->st_out, ev_done[k], 0));
+        SPK_CUDA(cudaMemcpyAsync(x + lo, dx + lo, sizeof(double) * cnt, cudaMemcpyDeviceToHost, s->st_out));
+    }
+    for (int k = 0; !one && k <= K; k++) {
         if (k < K) {
             cudaStream_t q = s->pipe_st[k];
             SPK_CUDA(cudaStreamWaitEvent(q, ev_in[k], 0));
@@ -1416,8 +1529,16 @@ long long chain_device_check() {
 #endif
 }
 
-// One solve through the chain path: phase 1 then phase 4 on stream st.
+// One solve through the chain path: one launch, or phase 1 then phase 4, on stream st.
 int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring) {
+    if (s->ov.len) {
+        SPK_TRY(launch_chain<false>(s, s->ov.d1.p, (int)s->ov.h1.size(), b, x, st));
+        if (prof) {
+            cudaEventRecord(s->ev[ring][1], st);
+            cudaEventRecord(s->ev[ring][2], st);
+        }
+        return SPK_OK;
+    }
     SPK_TRY(launch_chain<false>(s, s->d_ctasks1.p, s->nctasks1, b, x, st));
     if (prof) {
         cudaEventRecord(s->ev[ring][1], st);
@@ -1473,6 +1594,23 @@ int chain_tune(spk_system *s, const char *name, long long v) {
         return SPK_ERR_ARG;
     }
     const long long len = 32ll * ((v + 31) / 32);
+    if (plain && s->ov.len) {  // the one-launch solve takes any length
+        ChainPlan t;
+        SPK_TRY(build_overlap(s, len, t));
+        if (!t.len) {
+            set_error(SPK_ERR_ARG, "no start below tasks of %lld rows leaves them final", len);
+            return SPK_ERR_ARG;
+        }
+        SPK_CUDA(cudaDeviceSynchronize());
+        s->ov.release();
+        s->ov_host.release();
+        s->host_plan_tried = 0;
+        s->ov.d1.p = t.d1.p, s->ov.d1.n = t.d1.n, t.d1.p = nullptr;
+        s->ov.h1.swap(t.h1);
+        s->ov.len = t.len;
+        drop_pipeline();
+        return SPK_OK;
+    }
     ChainPlan fresh;
     const int keep_len = s->ch_len;
     s->ch_len = 0;  // so that build_plan builds the extra plan even at the plain length

@@ -2133,7 +2133,8 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
         set_error(SPK_ERR_STATE, "no preprocessed system");
         return SPK_ERR_STATE;
     }
-    if (!(s->chain_ok && (!ph || s->lean))) SPK_TRY(partition_ensure(s));  // the partition path below
+    const bool chains = (s->chain_ok || s->ov.len) && (!ph || s->lean);
+    if (!chains) SPK_TRY(partition_ensure(s));  // the partition path below
     double t0 = 0;
     auto lap = [&](int slot) {
         if (!ph) return;
@@ -2150,7 +2151,7 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
         if (s->ev_pending[ring]) SPK_TRY(collect_event_set(s, ring));
         cudaEventRecord(s->ev[ring][0], st);
     }
-    if (s->chain_ok && (!ph || s->lean)) {  // a compacted system has no other path (no phase times)
+    if (chains) {  // a compacted system has no other path (no phase times)
         SPK_TRY(chain_solve(s, b, x, st, prof, ring));
     } else if ((s->ell_ok || s->sw_ok) && !ph) {
         SPK_TRY((launch_tiles<1, double>(s, b, s->n, x, s->n, s->xbuf.p, st, prof, ring)));
