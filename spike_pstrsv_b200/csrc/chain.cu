@@ -61,6 +61,7 @@
 
 #include "spk_internal.cuh"
 #include "sweep.cuh"
+#include "sweep_rhs.cuh"
 
 namespace spk {
 
@@ -1039,6 +1040,7 @@ void chain_release(spk_system *s, bool keep_overlap = false) {
     if (!keep_overlap) {
         s->ov.release();
         s->ov_host.release();
+        s->ov_batch.release();
         s->ov_warm = 0;
     }
     s->host_plan_tried = 0;
@@ -1063,6 +1065,7 @@ int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra);
 long long overlap_rows(spk_system *s, int sms, int occ);
 long long overlap_warm(const spk_system *s);
 int build_overlap(spk_system *s, long long len, ChainPlan &out);
+long long batch_overlap_rows(const spk_system *s, int sms);
 
 // Build the chain layout, the chains' spikes and the two task lists; leaves
 // chain_ok = 0 (the partition-based solve) when truncation is off, the layout
@@ -1142,8 +1145,23 @@ int chain_prepare(spk_system *s) {
     lenb = std::max<long long>(lenb, s->ch_len);
     if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) lenb = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     if (lenb > s->ch_len) SPK_TRY(build_plan(s, lenb, reach, &s->cp_batch));
-    if (s->sw_ok) SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
+    if (s->sw_ok) {
+        SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
+        const long long lb = batch_overlap_rows(s, sms);
+        if (s->ov.len) SPK_TRY(build_overlap(s, lb, s->ov_batch));
+    }
     return SPK_OK;
+}
+
+// Rows per task of the batched one-launch solve: two tasks an SM once a task's own rows
+// outnumber the rows it walks before them, else one (two slow each other down by 1.1, with
+// 17 and more right-hand sides by 1.6).  FP64, one / two / three tasks: 32 right-hand sides,
+// 4,194,304 banded rows 1,767 / 1,446 / 1,630 us, 20,011 rows 127 / 185 / 210 us; 300,007 rows,
+// 21: 220 / 248 / 424 us, 12: 207 / 160 / 186 us, 4: 187 / 143 / 163 us.
+long long batch_overlap_rows(const spk_system *s, int sms) {
+    if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) return std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
+    const long long w = s->n / sms >= overlap_warm(s) ? 2 : 1;
+    return std::max(32ll, 32ll * ((s->n / (sms * w) + 31) / 32));
 }
 
 // Rows per task of the one-launch solve.  With w tasks an SM a task walks n / (sms w) +
@@ -1483,14 +1501,35 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
     return SPK_OK;
 }
 
-// Up to 32 right-hand sides (device, column-major) through the chain path:
+// Whether nk right-hand sides go in one launch on 16-row records (made here on first use),
+// and may then be added to X.
+bool chain_rhs_one(spk_system *s, int fp32, int nk) {
+    if (!s->ov_batch.len || rhs_sweep_prepare(s, fp32) != SPK_OK) return false;
+    return rhs_sweep_fits(s, fp32, nk);
+}
+
+// Up to 32 right-hand sides (device, column-major) through the chain path: one launch, or
 // phase 1 then phase 4 of the right-hand-side-parallel chain kernel, in T
 // (double, or float with the FP32 copy of the values).  X is FP64.
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st) {
+                    cudaStream_t st, int acc) {
     if (nk < 1 || nk > 32) {
         set_error(SPK_ERR_ARG, "chain batch of %d columns (1..32)", nk);
         return SPK_ERR_ARG;
+    }
+    if (chain_rhs_one(s, fp32, nk)) {
+        RhsSweep A = rhs_sweep_args(s, fp32, nk);
+        A.tasks = s->ov_batch.d1.p;
+        A.ntasks = (int)s->ov_batch.h1.size();
+        A.B = B;
+        A.ldb = ldb;
+        A.X = X;
+        A.ldx = ldx;
+        A.acc = acc;
+        A.rev_b = A.rev_x = s->uplo == 'L';
+        SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
+        s->launches++;
+        return SPK_OK;
     }
     const ChainPlan &bp = s->cp_batch;
     const bool own = bp.len > 0;  // the batched kernel's own chains
@@ -1594,7 +1633,7 @@ int chain_tune(spk_system *s, const char *name, long long v) {
         return SPK_ERR_ARG;
     }
     const long long len = 32ll * ((v + 31) / 32);
-    if (plain && s->ov.len) {  // the one-launch solve takes any length
+    if (plain ? s->ov.len : s->ov_batch.len) {  // the one-launch solves take any length
         ChainPlan t;
         SPK_TRY(build_overlap(s, len, t));
         if (!t.len) {
@@ -1602,13 +1641,16 @@ int chain_tune(spk_system *s, const char *name, long long v) {
             return SPK_ERR_ARG;
         }
         SPK_CUDA(cudaDeviceSynchronize());
-        s->ov.release();
-        s->ov_host.release();
-        s->host_plan_tried = 0;
-        s->ov.d1.p = t.d1.p, s->ov.d1.n = t.d1.n, t.d1.p = nullptr;
-        s->ov.h1.swap(t.h1);
-        s->ov.len = t.len;
-        drop_pipeline();
+        ChainPlan &to = plain ? s->ov : s->ov_batch;
+        to.release();
+        to.d1.p = t.d1.p, to.d1.n = t.d1.n, t.d1.p = nullptr;
+        to.h1.swap(t.h1);
+        to.len = t.len;
+        if (plain) {
+            s->ov_host.release();
+            s->host_plan_tried = 0;
+            drop_pipeline();
+        }
         return SPK_OK;
     }
     ChainPlan fresh;

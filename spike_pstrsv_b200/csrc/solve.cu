@@ -40,6 +40,7 @@
 #include "reduced.cuh"
 #include "spk_internal.cuh"
 #include "sweep.cuh"
+#include "sweep_rhs.cuh"
 
 namespace spk {
 
@@ -2006,6 +2007,40 @@ int launch_rhs(spk_system *s, int nk, const double *rhs, long long ldb, double *
     return SPK_OK;
 }
 
+// One Spike solve of nk right-hand sides on 16-row records (rhs_sweep_fits); work holds the
+// columns rounded up to a power of two.  acc: X += x.
+int launch_sweep_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx, void *work,
+                     cudaStream_t st, int acc) {
+    RhsSweep A = rhs_sweep_args(s, fp32, nk);
+    A.seg = 1;
+    A.B = B;
+    A.ldb = ldb;
+    A.rev_b = s->uplo == 'L';
+    if (s->redNec && s->ntasks1) {
+        A.tasks = s->d_tasks1.p;
+        A.ntasks = s->ntasks1;
+        A.X = work;
+        A.ldx = s->n;
+        A.out_work = 1;
+        SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
+        s->launches++;
+    }
+    if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, fp32, nk, work, st));
+    A.tasks = s->d_tasks2.p;
+    A.ntasks = s->ntasks2;
+    A.copies = s->d_copies.p;
+    A.ncopies = s->ncopies;
+    A.X = X;
+    A.ldx = ldx;
+    A.out_work = 0;
+    A.acc = acc;
+    A.rev_x = s->uplo == 'L';
+    A.pre = work;
+    SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
+    s->launches++;
+    return SPK_OK;
+}
+
 // Coupling reach of the ELL copy (computed once).
 int ensure_reach(spk_system *s) {
     if (s->ell_reach >= 0) return SPK_OK;
@@ -2302,13 +2337,13 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
     SPK_CUDA(cudaGetDevice(&dev0));
     SPK_CUDA(cudaDeviceGetAttribute(&sms0, cudaDevAttrMultiProcessorCount, dev0));
     const bool part_wide = std::min(s->redNec ? s->ntasks1 : s->ntasks2, s->ntasks2) >= 2 * sms0;
-    // FP64: the chain kernel (faster than the partition kernels at every partition
-    // count measured); FP32 + refinement: the chain kernel when the partitions give
-    // too few tasks to fill the GPU
+    // the chain kernels, faster than the partition kernels at every partition count measured
+    // (4,194,304 banded rows in 1,024 partitions, 32 right-hand sides: FP64 1,445 against 3,727 us);
+    // FP32 + refinement without 16-row records: when the partitions give too few tasks to fill the GPU
     const char *cb = getenv("SPK_CHAIN_BATCH");  // 1: always the chain kernels, 0: never
     const bool use_chain =
         s->chain_ok && (s->lean || (s->batch_path >= 0 ? s->batch_path == 1
-                                                       : (cb ? cb[0] == '1' : (mode == 0 || !part_wide))));
+                                                       : (cb ? cb[0] == '1' : (mode == 0 || s->ov_batch.len || !part_wide))));
     if (!use_chain) SPK_TRY(partition_ensure(s));
     if (use_chain) {
         // the chain tasks fill the GPU whatever the partition count: every group
@@ -2339,6 +2374,10 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                         if ((tol >= 0 && r <= tol) || it == maxit) break;
                     }
                     if (it == maxit) break;
+                    if (chain_rhs_one(s, 1, K)) {
+                        SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, Xg, ldx, st, 1));
+                        continue;
+                    }
                     SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, dbuf_p, n, st));
                     k_axpy<<<dim3(148, K), 256, 0, st>>>(s->n, K, dbuf_p, Xg, ldx);
                     SPK_CUDA(cudaGetLastError());
@@ -2353,8 +2392,44 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
         if (resid || (mode != 0 && tol >= 0)) SPK_TRY(check_device_error(s));
         return SPK_OK;
     }
+    if (mode == 1 || nrhs > 1) SPK_TRY(rhs_sweep_prepare(s, mode));
     for (int g = 0; g < nrhs;) {
         const int left = nrhs - g;
+        const int Ks = std::min(left, 32);
+        if ((Ks > 1 || mode == 1) && rhs_sweep_fits(s, mode, Ks)) {
+            int cols = 1;
+            while (cols < Ks) cols <<= 1;
+            const size_t wbytes = ((mode ? sizeof(float) : sizeof(double)) * cols * n + 255) / 256 * 256;
+            const bool red64 = mode == 1 && s->redNec && s->nkept;
+            SPK_TRY(work_for(wbytes + (red64 ? red_bytes : 0)));
+            s->red_scratch = !red64 ? nullptr
+                             : s->ext_ws ? (double *)(s->ext_ws + col_bytes * (1 + need_r + need_d))
+                                         : (double *)(work_p + wbytes);
+            struct ClearRed {
+                spk_system *s;
+                ~ClearRed() { s->red_scratch = nullptr; }
+            } clear_red{s};
+            const double *Bg = B + g * ldb;
+            double *Xg = X + g * ldx;
+            SPK_TRY(launch_sweep_rhs(s, mode, Ks, Bg, ldb, Xg, ldx, work_p, st, 0));
+            int it = 0;
+            double r = -1.0;
+            for (; mode == 1 || resid; it++) {
+                const bool check = (mode == 1 && tol >= 0) || (resid && (mode == 0 || it == maxit));
+                if (mode == 1 && tol < 0 && it == maxit && !resid) break;
+                SPK_TRY(residual(s, Ks, Xg, ldx, Bg, ldb, rbuf_p, n, st, check));
+                if (check) {
+                    SPK_TRY(scaled_residual(s, Ks, st, &r));
+                    if ((tol >= 0 && r <= tol) || it == maxit) break;
+                }
+                if (mode == 0 || it == maxit) break;
+                SPK_TRY(launch_sweep_rhs(s, 1, Ks, rbuf_p, n, Xg, ldx, work_p, st, 1));
+            }
+            if (mode == 1) max_it = std::max(max_it, it);
+            if (!(r < 0)) worst = worst_of(worst, r);
+            g += Ks;
+            continue;
+        }
         // 17..32 columns: one right-hand-side-parallel pass (work holds 32 columns);
         // fewer (or few tasks): the tile solver in power-of-two groups
         const int K = (wide_ok && left > 16) ? std::min(left, 32)

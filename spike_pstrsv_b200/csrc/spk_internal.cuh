@@ -192,13 +192,17 @@ struct spk_system {
     spk::ChainPlan cp_batch;  // the batched kernel's own chains (longer; built at preprocessing)
     spk::ChainPlan cp_host;   // the host-array pipeline's chains (shorter; built on first use)
     // the one-launch solve on 16-row records: tasks that start ov_warm rows below their own
-    spk::ChainPlan ov, ov_host;  // ov_host: the host-array pipeline's, where ov's are too long
+    spk::ChainPlan ov, ov_host, ov_batch;  // ov_batch: the batched solve's; ov_host: the host-array pipeline's, where ov's are too long
     int ov_warm = 0;
     int batch_path = -1;      // spk_tune "batch_path": 1 chain kernels, 0 partition kernels, -1 automatic
     // 16-row records of U for the one-right-hand-side solves (sweep.cu)
     int sw_ok = 0, sw_win = 0, sw_reach = 0, sw_wide = 0, sw_slots = 0, sw_stage = 0;
     spk::DBuf<unsigned char> sw_rec;
     spk::DBuf<int2> sw_hdr;
+    // the same for many right-hand sides (sweep_rhs.cu; [0] FP64, [1] FP32; made on first use)
+    int rs_ok[2] = {0, 0}, rs_bytes[2] = {0, 0}, rs_groups = 0, rs_extras = 0;
+    spk::DBuf<unsigned char> rs_rec[2];
+    spk::DBuf<int2> rs_hdr[2];
     spk::DBuf<int2> d_copies;  // phase 3+4: row ranges that keep their phase-1 values
     int ncopies = 0;
     // wall milliseconds of the last preprocessing: the reference's steps, first
@@ -268,8 +272,9 @@ int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool
 int chain_solve_host(spk_system *s, const double *b, double *x, double *db, double *dx);
 long long chain_device_check();
 int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *b, double *x, cudaStream_t st);
+bool chain_rhs_one(spk_system *s, int fp32, int nk);
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st);
+                    cudaStream_t st, int acc = 0);
 int check_device_error(spk_system *s);
 int collect_phase_times(spk_system *s);
 int collect_event_set(spk_system *s, int k);

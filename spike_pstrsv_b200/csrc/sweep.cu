@@ -46,6 +46,7 @@
 #include <set>
 
 #include "sweep.cuh"
+#include "sweep_rhs.cuh"
 
 namespace spk {
 
@@ -366,12 +367,14 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
         }
         return;
     }
-    // x of rows [r0, r0 + count) into the window (zero past the matrix or without pre)
+    // x of rows [r0, r0 + count) into the window (zero past the matrix or without pre); of what no
+    // row reads, the row after a cut tile is zeroed too: unused slots point there
     const unsigned maskb = 8u * (unsigned)(A.win - 1);
     auto load_window = [&](int r0, int count) {
-        for (int k = lane; k < count; k += 32) {
+        for (int k = lane; k < max(A.reach, 17); k += 32) {
+            if (k >= count && k < A.reach) continue;
             const int r = r0 + k;
-            const double v = A.pre && r < A.n ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
+            const double v = A.pre && k < count && r < A.n ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
             const unsigned at = M.win + ((8u * (unsigned)r) & maskb);
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + 8 * A.win), "d"(v) : "memory");
@@ -414,10 +417,13 @@ __device__ __forceinline__ int first_from(const int *__restrict__ ja, int b, int
     return b;
 }
 
-// Per tile: slots per lane that its longest row needs (two lanes a row; even), and the
-// matrix's reach.  A half warp per tile.
+// Per tile: slots per lane that its longest row needs (two lanes a row; even); the matrix's
+// reach, and a histogram of the rows' outside columns.  A half warp per tile.
 __global__ void k_sweep_count(int n, int ntiles, const int *__restrict__ ia, const int *__restrict__ ja,
-                              int *__restrict__ slots, int *__restrict__ reach) {
+                              int *__restrict__ slots, int *__restrict__ reach, int *__restrict__ hist) {
+    __shared__ int sh[2 * kMaxSlots + 1];
+    for (int i = threadIdx.x; i <= 2 * kMaxSlots; i += blockDim.x) sh[i] = 0;
+    __syncthreads();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = r >> 4;
     int out = 0, d = 0;
@@ -425,6 +431,7 @@ __global__ void k_sweep_count(int n, int ntiles, const int *__restrict__ ia, con
         const int b = ia[r], e = ia[r + 1];
         out = e - first_from(ja, b, e, 16 * j + 16);
         d = ja[e - 1] - r;
+        atomicAdd(&sh[min(out, 2 * kMaxSlots)], 1);
     }
 #pragma unroll
     for (int o = 8; o; o >>= 1) out = max(out, __shfl_xor_sync(kFull, out, o, 16));
@@ -432,6 +439,9 @@ __global__ void k_sweep_count(int n, int ntiles, const int *__restrict__ ia, con
     for (int o = 16; o; o >>= 1) d = max(d, __shfl_xor_sync(kFull, d, o));
     if ((r & 15) == 0 && j < ntiles) slots[j] = ((out + 1) / 2 + 1) & ~1;
     if ((threadIdx.x & 31) == 0) atomicMax(reach, d);
+    __syncthreads();
+    for (int i = threadIdx.x; i <= 2 * kMaxSlots; i += blockDim.x)
+        if (sh[i]) atomicAdd(&hist[i], sh[i]);
 }
 
 // The records, a warp per tile.
@@ -525,17 +535,10 @@ int allow_smem(K kern) {
 
 }  // namespace
 
-void sweep_release(spk_system *s) {
-    s->sw_ok = 0;
-    s->sw_rec.release();
-    s->sw_hdr.release();
-    s->d_copies.release();
-    s->ncopies = 0;
-}
-
 // The records of U; sw_ok = 0 (the row-by-row kernels run) when a row reaches past the
 // window, a row has more than 2 kMaxSlots of them, or W grows past kGrowth.
 int sweep_prepare(spk_system *s) {
+    rhs_sweep_release(s);
     s->sw_ok = 0;
     s->sw_rec.release();
     s->sw_hdr.release();
@@ -543,15 +546,16 @@ int sweep_prepare(spk_system *s) {
     if (no && no[0] == '1') return SPK_OK;
     const int n = s->n, nt = (n + 15) / 16;
     cudaStream_t st = s->stream;
-    std::vector<int> hs(nt + 1);
+    constexpr int kTail = 1 + 2 * kMaxSlots + 1;  // after the tiles: the reach, the histogram
+    std::vector<int> hs(nt + kTail);
     std::vector<int2> hd(nt);
     {
         DBuf<int> d(st);
-        SPK_TRY(d.alloc(nt + 1));
-        SPK_CUDA(cudaMemsetAsync(d.p + nt, 0, sizeof(int), st));
-        k_sweep_count<<<(nt * 16 + 255) / 256, 256, 0, st>>>(n, nt, s->uia.p, s->uja.p, d.p, d.p + nt);
+        SPK_TRY(d.alloc(nt + kTail));
+        SPK_CUDA(cudaMemsetAsync(d.p + nt, 0, sizeof(int) * kTail, st));
+        k_sweep_count<<<(nt * 16 + 255) / 256, 256, 0, st>>>(n, nt, s->uia.p, s->uja.p, d.p, d.p + nt, d.p + nt + 1);
         SPK_CUDA(cudaGetLastError());
-        SPK_CUDA(cudaMemcpyAsync(hs.data(), d.p, sizeof(int) * (nt + 1), cudaMemcpyDeviceToHost, st));
+        SPK_CUDA(cudaMemcpyAsync(hs.data(), d.p, sizeof(int) * (nt + kTail), cudaMemcpyDeviceToHost, st));
         SPK_CUDA(cudaStreamSynchronize(st));
     }
     const int reach = hs[nt];
@@ -612,6 +616,7 @@ int sweep_prepare(spk_system *s) {
     s->sw_slots = S0;
     s->sw_stage = most + 128;
     s->sw_ok = 1;
+    rhs_sweep_choose(s, hs.data() + nt + 1, 2 * kMaxSlots);
     return SPK_OK;
 }
 

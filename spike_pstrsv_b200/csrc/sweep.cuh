@@ -30,7 +30,6 @@ struct SweepArgs {
 };
 
 int sweep_prepare(spk_system *s);
-void sweep_release(spk_system *s);
 int sweep_copies(spk_system *s, const std::vector<SegTask> &t2);
 // Arguments that depend on the system alone.
 SweepArgs sweep_args(const spk_system *s);
