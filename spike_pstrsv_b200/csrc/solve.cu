@@ -35,6 +35,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <ctime>
+#include <memory>
 #include <mutex>
 
 #include "reduced.cuh"
@@ -1877,8 +1878,7 @@ int partition_ensure(spk_system *s) {
 namespace {
 
 // Phase 1 (into work, U order) and phase 3+4 of one right-hand side on 16-row records.
-int sweep_phase(spk_system *s, bool phase4, const double *rhs, double *xo, double *work, bool dependent,
-                cudaStream_t st) {
+SweepArgs sweep_seg_args(const spk_system *s, bool phase4, const double *rhs, double *xo, double *work) {
     SweepArgs A = sweep_args(s);
     A.b = rhs;
     A.rev_b = s->uplo == 'L';
@@ -1896,7 +1896,12 @@ int sweep_phase(spk_system *s, bool phase4, const double *rhs, double *xo, doubl
         A.x = work;
     }
     A.seg = 1;
-    SPK_TRY(sweep_launch(s, A, dependent, st));
+    return A;
+}
+
+int sweep_phase(spk_system *s, bool phase4, const double *rhs, double *xo, double *work, bool dependent,
+                cudaStream_t st) {
+    SPK_TRY(sweep_launch(s, sweep_seg_args(s, phase4, rhs, xo, work), dependent, st));
     s->launches++;
     return SPK_OK;
 }
@@ -2007,36 +2012,44 @@ int launch_rhs(spk_system *s, int nk, const double *rhs, long long ldb, double *
     return SPK_OK;
 }
 
-// One Spike solve of nk right-hand sides on 16-row records (rhs_sweep_fits); work holds the
-// columns rounded up to a power of two.  acc: X += x.
-int launch_sweep_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx, void *work,
-                     cudaStream_t st, int acc) {
+// Phase 1 (into work, U order) and phase 3+4 of nk right-hand sides on 16-row records
+// (rhs_sweep_fits).  acc: X += x.
+RhsSweep rhs_seg_args(const spk_system *s, int fp32, int nk, bool phase4, const double *B, long long ldb, double *X,
+                      long long ldx, void *work, int acc) {
     RhsSweep A = rhs_sweep_args(s, fp32, nk);
     A.seg = 1;
     A.B = B;
     A.ldb = ldb;
     A.rev_b = s->uplo == 'L';
-    if (s->redNec && s->ntasks1) {
+    if (phase4) {
+        A.tasks = s->d_tasks2.p;
+        A.ntasks = s->ntasks2;
+        A.copies = s->d_copies.p;
+        A.ncopies = s->ncopies;
+        A.X = X;
+        A.ldx = ldx;
+        A.acc = acc;
+        A.rev_x = s->uplo == 'L';
+        A.pre = work;
+    } else {
         A.tasks = s->d_tasks1.p;
         A.ntasks = s->ntasks1;
         A.X = work;
         A.ldx = s->n;
         A.out_work = 1;
-        SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
+    }
+    return A;
+}
+
+// One Spike solve of nk right-hand sides; work holds the columns rounded up to a power of two.
+int launch_sweep_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx, void *work,
+                     cudaStream_t st, int acc) {
+    if (s->redNec && s->ntasks1) {
+        SPK_TRY(rhs_sweep_launch(s, rhs_seg_args(s, fp32, nk, false, B, ldb, X, ldx, work, 0), fp32, st));
         s->launches++;
     }
     if (s->redNec && s->nkept) SPK_TRY(reduced_solve(s, fp32, nk, work, st));
-    A.tasks = s->d_tasks2.p;
-    A.ntasks = s->ntasks2;
-    A.copies = s->d_copies.p;
-    A.ncopies = s->ncopies;
-    A.X = X;
-    A.ldx = ldx;
-    A.out_work = 0;
-    A.acc = acc;
-    A.rev_x = s->uplo == 'L';
-    A.pre = work;
-    SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
+    SPK_TRY(rhs_sweep_launch(s, rhs_seg_args(s, fp32, nk, true, B, ldb, X, ldx, work, acc), fp32, st));
     s->launches++;
     return SPK_OK;
 }
@@ -2639,19 +2652,18 @@ int clobber_rhs(spk_system *s, const double *x, double *b, cudaStream_t st) {
 
 // ---- many systems in one captured launch sequence (spk_group) --------------------
 //
-// Every system's right-hand sides are split into width classes K in
-// {16, 8, 4, 2, 1} ("virtual systems": one system, K columns).  Per class, one
-// k_tile_multi launch runs the phase-1 tasks of all its virtual systems from a
-// flat work list (longest tasks first), one launch per column block width their
-// reduced solves (reduced.cu; a cluster per system and column block), one k_tile_multi launch their
-// phase 3+4 tasks; FP32 + refinement adds k_residual_multi and k_axpy_multi
-// over flat row-block lists.  The whole sequence is captured once into a CUDA
-// graph and replayed by spk_group_solve.
+// Every system's right-hand sides are split into widths K in {16, 8, 4, 2, 1}
+// ("virtual systems": one system, K columns), and those into classes that one kernel
+// serves (width, and 16-row records of one shape or the row-by-row tiles).  Per class,
+// one launch runs the phase-1 tasks of all its virtual systems from a flat work list
+// (longest tasks first), one per column block width their reduced solves (reduced.cu; a
+// cluster per system and column block), one their phase 3+4 tasks; FP32 + refinement
+// adds k_residual_multi, and k_axpy_multi on the tiles, over flat row-block lists.  The
+// whole sequence, a branch per class, is captured once into a CUDA graph and replayed
+// by spk_group_solve.
 
 namespace spk {
 namespace {
-
-constexpr int kGroupK[5] = {16, 8, 4, 2, 1};
 
 struct GroupVS {
     spk_system *s;
@@ -2666,9 +2678,29 @@ struct GroupVS {
     double *red;  // FP32 batches: the FP64 reduced unknowns ([K][nRed])
 };
 
+// How a virtual system's tasks run: on 16-row records (sweep.cu for one FP64 column, with the
+// common slots and offset width; sweep_rhs.cu otherwise, with the launch class), or on the
+// row-by-row tile kernels.
+struct GroupKind {
+    enum { kTiles, kSweep, kRhs } path = kTiles;
+    int id = 0;
+    bool operator==(const GroupKind &o) const { return path == o.path && id == o.id; }
+};
+
+GroupKind kind_of(const spk_system *s, int K, int fp32) {
+    if (K == 1 && !fp32 && s->sw_ok) return GroupKind{GroupKind::kSweep, 2 * s->sw_slots + s->sw_wide};
+    if (rhs_sweep_fits(s, fp32, K)) return GroupKind{GroupKind::kRhs, rhs_sweep_class(s, fp32, K)};
+    return GroupKind{};
+}
+
+// Virtual systems of one width and kind: one launch per phase.
 struct GroupClass {
     int K = 0;
+    GroupKind kind;
     DBuf<TileArgs> a1, a4, c1, c4;  // solve and correction-solve arguments (phase 1, phase 3+4)
+    DBuf<SweepArgs> s1, s4;
+    DBuf<RhsSweep> r1, r4, e1, e4;  // e: corrections, added to X
+    size_t smem = 0;
     DBuf<int2> w1, w4, vw;
     RedPlan red;  // the class's reduced solves
     DBuf<VecArgs> va;
@@ -2683,7 +2715,7 @@ struct spk_group {
     int mode = 0, iters = 0;
     std::vector<spk_system *> sys;
     std::vector<spk::GroupVS> vs;
-    spk::GroupClass cls[5];
+    std::vector<std::unique_ptr<spk::GroupClass>> cls;
     spk::DBuf<char> pool;
     spk::DBuf<unsigned long long> norms;
     long long norm_cols = 0;
@@ -2691,6 +2723,7 @@ struct spk_group {
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;
     int rc = SPK_OK;  // first failed launch of the capture
+    std::vector<cudaStream_t> branches;  // of the capture
 };
 
 namespace spk {
@@ -2739,16 +2772,32 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
     std::vector<TileArgs> a1, a4, c1, c4;
     std::vector<RedMember> red;
     std::vector<VecArgs> va;
+    std::vector<SweepArgs> s1, s4;
+    std::vector<RhsSweep> r1, r4, e1, e4;
     std::vector<std::pair<long long, int2>> w1, w4;
     std::vector<int2> vw;
     for (size_t i = 0; i < c.vs.size(); i++) {
         const GroupVS &v = g->vs[c.vs[i]];
         spk_system *s = v.s;
-        a1.push_back(make_args(v, fp32, false, v.B, v.ldb, nullptr, 0));
-        a4.push_back(make_args(v, fp32, true, v.B, v.ldb, v.X, v.ldx));
-        if (fp32) {
-            c1.push_back(make_args(v, true, false, v.R, s->n, nullptr, 0));
-            c4.push_back(make_args(v, true, true, v.R, s->n, v.D, s->n));
+        if (c.kind.path == GroupKind::kSweep) {
+            s1.push_back(sweep_seg_args(s, false, v.B, nullptr, (double *)v.work));
+            s4.push_back(sweep_seg_args(s, true, v.B, v.X, (double *)v.work));
+            c.smem = std::max(c.smem, sweep_smem(s));
+        } else if (c.kind.path == GroupKind::kRhs) {
+            r1.push_back(rhs_seg_args(s, fp32, c.K, false, v.B, v.ldb, nullptr, 0, v.work, 0));
+            r4.push_back(rhs_seg_args(s, fp32, c.K, true, v.B, v.ldb, v.X, v.ldx, v.work, 0));
+            if (fp32) {
+                e1.push_back(rhs_seg_args(s, 1, c.K, false, v.R, s->n, nullptr, 0, v.work, 0));
+                e4.push_back(rhs_seg_args(s, 1, c.K, true, v.R, s->n, v.X, v.ldx, v.work, 1));
+            }
+            c.smem = std::max(c.smem, rhs_sweep_smem(s, fp32, c.K));
+        } else {
+            a1.push_back(make_args(v, fp32, false, v.B, v.ldb, nullptr, 0));
+            a4.push_back(make_args(v, fp32, true, v.B, v.ldb, v.X, v.ldx));
+            if (fp32) {
+                c1.push_back(make_args(v, true, false, v.R, s->n, nullptr, 0));
+                c4.push_back(make_args(v, true, true, v.R, s->n, v.D, s->n));
+            }
         }
         if (s->redNec && s->ntasks1)
             for (int t = 0; t < s->ntasks1; t++) {
@@ -2759,6 +2808,8 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
             const SegTask &q = t4[v.sys][t];
             w4.push_back({(long long)(q.hi - q.lo) + (q.tail - q.hi), make_int2((int)i, t)});
         }
+        if (c.kind.path != GroupKind::kTiles)
+            for (int t = 0; t < s->ncopies; t++) w4.push_back({0, make_int2((int)i, s->ntasks2 + t)});
         if (s->redNec && s->nkept) red.push_back(RedMember{s, v.work, v.red});
         VecArgs a{};
         a.n = s->n;
@@ -2789,11 +2840,17 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
         SPK_TRY(upload_vec(c.c1, c1));
         SPK_TRY(upload_vec(c.c4, c4));
     }
-    const std::vector<int2> s1 = sorted(w1), s4 = sorted(w4);
-    SPK_TRY(upload_vec(c.w1, s1));
-    SPK_TRY(upload_vec(c.w4, s4));
-    c.n1 = (int)s1.size();
-    c.n4 = (int)s4.size();
+    SPK_TRY(upload_vec(c.s1, s1));
+    SPK_TRY(upload_vec(c.s4, s4));
+    SPK_TRY(upload_vec(c.r1, r1));
+    SPK_TRY(upload_vec(c.r4, r4));
+    SPK_TRY(upload_vec(c.e1, e1));
+    SPK_TRY(upload_vec(c.e4, e4));
+    const std::vector<int2> o1 = sorted(w1), o4 = sorted(w4);
+    SPK_TRY(upload_vec(c.w1, o1));
+    SPK_TRY(upload_vec(c.w4, o4));
+    c.n1 = (int)o1.size();
+    c.n4 = (int)o4.size();
     SPK_TRY(red_plan_build(c.red, red, c.K, fp32));
     SPK_TRY(upload_vec(c.va, va));
     SPK_TRY(upload_vec(c.vw, vw));
@@ -2803,17 +2860,27 @@ int build_class(spk_group *g, GroupClass &c, const std::vector<std::vector<SegTa
 
 template <int K, typename T>
 void enqueue_solve(spk_group *g, GroupClass &c, bool correction, cudaStream_t st) {
-    const TileArgs *p1 = correction ? c.c1.p : c.a1.p;
-    const TileArgs *p4 = correction ? c.c4.p : c.a4.p;
-    if (c.n1) {
-        k_tile_multi<false, K, T, T><<<c.n1, 32, 0, st>>>(p1, c.w1.p);
+    constexpr int fp32 = sizeof(T) == 4;
+    auto keep = [&](int rc) {
+        if (rc != SPK_OK && g->rc == SPK_OK) g->rc = rc;
+    };
+    auto phase = [&](bool last, const int2 *work, int count) {
+        if (!count) return;
+        if (c.kind.path == GroupKind::kSweep) {
+            keep(sweep_launch_multi(last ? c.s4.p : c.s1.p, work, count, c.kind.id / 2, c.kind.id % 2, c.smem, st));
+        } else if (c.kind.path == GroupKind::kRhs) {
+            const RhsSweep *tab = correction ? (last ? c.e4.p : c.e1.p) : (last ? c.r4.p : c.r1.p);
+            keep(rhs_sweep_launch_multi(tab, work, count, c.kind.id, fp32, c.smem, st));
+        } else if (last) {
+            k_tile_multi<true, K, T, double><<<count, 32, 0, st>>>(correction ? c.c4.p : c.a4.p, work);
+        } else {
+            k_tile_multi<false, K, T, T><<<count, 32, 0, st>>>(correction ? c.c1.p : c.a1.p, work);
+        }
         g->kernels++;
-    }
-    if (const int rc = red_plan_launch(c.red, st, &g->kernels); rc != SPK_OK) g->rc = rc;
-    if (c.n4) {
-        k_tile_multi<true, K, T, double><<<c.n4, 32, 0, st>>>(p4, c.w4.p);
-        g->kernels++;
-    }
+    };
+    phase(false, c.w1.p, c.n1);
+    keep(red_plan_launch(c.red, st, &g->kernels));
+    phase(true, c.w4.p, c.n4);
 }
 
 template <int K>
@@ -2826,22 +2893,40 @@ void enqueue_class(spk_group *g, GroupClass &c, cudaStream_t st) {
     for (int it = 0; it < g->iters; it++) {
         k_residual_multi<K><<<c.nvw, 256, 0, st>>>(c.va.p, c.vw.p, 0);
         enqueue_solve<K, float>(g, c, true, st);
+        g->kernels++;
+        if (c.kind.path == GroupKind::kRhs) continue;  // added by the solve
         k_axpy_multi<K><<<c.nvw, 256, 0, st>>>(c.va.p, c.vw.p);
-        g->kernels += 2;
+        g->kernels++;
     }
 }
 
-void enqueue_all(spk_group *g, cudaStream_t st) {
-    for (auto &c : g->cls) {
-        if (c.vs.empty()) continue;
+// The classes have no data in common: each runs on a branch of its own, forked from and
+// joined to the captured stream (their phases are chains of small launches, which leave
+// most of the GPU idle one after another).
+int enqueue_all(spk_group *g, cudaStream_t st) {
+    cudaEvent_t fork, join;
+    SPK_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    SPK_CUDA(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    SPK_CUDA(cudaEventRecord(fork, st));
+    for (auto &p : g->cls) {
+        GroupClass &c = *p;
+        cudaStream_t q;
+        SPK_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+        g->branches.push_back(q);
+        SPK_CUDA(cudaStreamWaitEvent(q, fork, 0));
         switch (c.K) {
-            case 16: enqueue_class<16>(g, c, st); break;
-            case 8: enqueue_class<8>(g, c, st); break;
-            case 4: enqueue_class<4>(g, c, st); break;
-            case 2: enqueue_class<2>(g, c, st); break;
-            default: enqueue_class<1>(g, c, st); break;
+            case 16: enqueue_class<16>(g, c, q); break;
+            case 8: enqueue_class<8>(g, c, q); break;
+            case 4: enqueue_class<4>(g, c, q); break;
+            case 2: enqueue_class<2>(g, c, q); break;
+            default: enqueue_class<1>(g, c, q); break;
         }
+        SPK_CUDA(cudaEventRecord(join, q));
+        SPK_CUDA(cudaStreamWaitEvent(st, join, 0));
     }
+    SPK_CUDA(cudaEventDestroy(fork));
+    SPK_CUDA(cudaEventDestroy(join));
+    return SPK_OK;
 }
 
 }  // namespace
@@ -2889,6 +2974,8 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
             return fail(SPK_ERR_STATE);
         }
         if (const int rc = partition_ensure(s); rc != SPK_OK) return fail(rc);
+        if (mode == 1 || nrhs[i] > 1)
+            if (const int rc = rhs_sweep_prepare(s, mode); rc != SPK_OK) return fail(rc);
         if (mode == 1) {
             int rc = ensure_fp32(s);
             if (rc == SPK_OK) rc = ensure_residual(s);
@@ -2948,13 +3035,21 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
             v.red = (double *)(g->pool.p + (intptr_t)v.red);
         }
     }
-    for (int c = 0; c < 5; c++) g->cls[c].K = kGroupK[c];
-    for (int i = 0; i < (int)g->vs.size(); i++)
-        for (int c = 0; c < 5; c++)
-            if (g->vs[i].K == kGroupK[c]) g->cls[c].vs.push_back(i);
+    for (int i = 0; i < (int)g->vs.size(); i++) {
+        const GroupKind kind = kind_of(g->vs[i].s, g->vs[i].K, mode);
+        GroupClass *c = nullptr;
+        for (auto &p : g->cls)
+            if (p->K == g->vs[i].K && p->kind == kind) c = p.get();
+        if (!c) {
+            g->cls.emplace_back(new GroupClass);
+            c = g->cls.back().get();
+            c->K = g->vs[i].K;
+            c->kind = kind;
+        }
+        c->vs.push_back(i);
+    }
     for (auto &c : g->cls) {
-        if (c.vs.empty()) continue;
-        const int rc = build_class(g, c, t1, t4);
+        const int rc = build_class(g, *c, t1, t4);
         if (rc != SPK_OK) return fail(rc);
     }
     // capture the launch sequence
@@ -2963,8 +3058,11 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
         set_error(SPK_ERR_CUDA, "cudaStreamBeginCapture failed (a legacy default stream cannot be captured)");
         return fail(SPK_ERR_CUDA);
     }
-    enqueue_all(g, st);
+    const int enq = enqueue_all(g, st);
+    if (g->rc == SPK_OK) g->rc = enq;
     cudaError_t e = cudaStreamEndCapture(st, &g->graph);
+    for (cudaStream_t q : g->branches) cudaStreamDestroy(q);
+    g->branches.clear();
     if (g->rc != SPK_OK) {
         (void)cudaGetLastError();
         return fail(g->rc);
@@ -3001,8 +3099,8 @@ int spk_group_residual(spk_group *g, void *stream, double *worst) {
         for (auto &v : g->vs) maxkn += (long long)v.K * v.s->n;
         SPK_TRY(scratch.alloc(std::max<long long>(maxkn, 1)));
         long long off = 0;
-        for (auto &c : g->cls) {
-            if (c.vs.empty()) continue;
+        for (auto &p : g->cls) {
+            GroupClass &c = *p;
             std::vector<VecArgs> va(c.vs.size());
             SPK_CUDA(cudaMemcpy(va.data(), c.va.p, sizeof(VecArgs) * va.size(), cudaMemcpyDeviceToHost));
             for (size_t i = 0; i < va.size(); i++) {
@@ -3013,8 +3111,8 @@ int spk_group_residual(spk_group *g, void *stream, double *worst) {
         }
     }
     SPK_CUDA(cudaMemsetAsync(g->norms.p, 0, sizeof(unsigned long long) * 3 * g->norm_cols, st));
-    for (auto &c : g->cls) {
-        if (c.vs.empty()) continue;
+    for (auto &p : g->cls) {
+        GroupClass &c = *p;
         switch (c.K) {
             case 16: k_residual_multi<16><<<c.nvw, 256, 0, st>>>(c.va.p, c.vw.p, 1); break;
             case 8: k_residual_multi<8><<<c.nvw, 256, 0, st>>>(c.va.p, c.vw.p, 1); break;
@@ -3048,7 +3146,7 @@ long long spk_group_info(const spk_group *g, const char *name) {
     if (!strcmp(name, "virtual_systems")) return (long long)g->vs.size();
     if (!strcmp(name, "columns")) return g->norm_cols;
     long long items = 0;
-    for (auto &c : g->cls) items += c.n1 + c.n4;
+    for (auto &c : g->cls) items += c->n1 + c->n4;
     if (!strcmp(name, "task_items")) return items;
     if (!strcmp(name, "pool_bytes")) return (long long)g->pool.n;
     return -1;
