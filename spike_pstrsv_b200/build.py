@@ -19,7 +19,7 @@ LIB = os.path.join(HERE, "libspike_pstrsv_b200.so")
 COMPAT_LIB = os.path.join(HERE, "libspike_pstrsv_mklcompat.so")
 COMPAT_SRC = "mklcompat.cu"
 
-SOURCES = ["preproc.cu", "solve.cu", "reduced.cu", "sweep.cu", "sweep_rhs.cu", "chain.cu", "capi.cu", "server.cu", "mtx.cu", "reorder.cu"]
+SOURCES = ["preproc.cu", "solve.cu", "reduced.cu", "sweep.cu", "sweep_rhs.cu", "residual.cu", "chain.cu", "capi.cu", "server.cu", "mtx.cu", "reorder.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-shared", "-Xcompiler", "-fPIC,-O2",
          "-Xptxas", "-warn-spills"]

@@ -1840,6 +1840,8 @@ int solve_prepare(spk_system *s) {
                     !(no_ell && no_ell[0] == '1');
         if (s->ell_ok) {
             ptr[ntiles] = (int)tot;
+            s->ell_chunk = 0;
+            for (int j = 0; j < ntiles; j += 4) s->ell_chunk = std::max(s->ell_chunk, ptr[std::min(j + 4, ntiles)] - ptr[j]);
             SPK_TRY(upload(s->ell_ptr, ptr));
             SPK_TRY(s->ell_val.alloc(std::max<long long>(tot, 1)));
             SPK_TRY(s->ell_col.alloc(std::max<long long>(tot, 1)));
@@ -2120,6 +2122,7 @@ inline double worst_of(double w, double v) { return (v > w || v != v) ? v : w; }
 int residual(spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,
              long long ldr, cudaStream_t st, bool norms) {
     if (norms) SPK_CUDA(cudaMemsetAsync(s->d_norms.p, 0, sizeof(unsigned long long) * 3 * K, st));
+    if (residual_fits(s, K)) return residual_launch(s, K, X, ldx, B, ldb, R, ldr, norms ? s->d_norms.p : nullptr, st);
     // the fixed-width kernels cover 1, 2, 4, 8 and 16 columns; other widths (the
     // chain path batches any count up to 32) take the any-width kernel, which
     // touches only columns < K
@@ -2310,11 +2313,10 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
     const size_t col_bytes = ((size_t)32 * n * sizeof(double) + 255) / 256 * 256;
     char *work_p = nullptr;
     double *rbuf_p = nullptr, *dbuf_p = nullptr;
-    if (mode == 1) {
-        SPK_TRY(ensure_fp32(s));
+    if (need_r) {
         SPK_TRY(ensure_reach(s));
+        SPK_TRY(ensure_residual(s));
     }
-    if (need_r) SPK_TRY(ensure_residual(s));
     // FP32 batches: the FP64 reduced unknowns (32 columns), after the other blocks
     const size_t red_bytes = mode == 1 ? (size_t)32 * s->nRed * sizeof(double) : 0;
     if (s->ext_ws) {
@@ -2464,6 +2466,7 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                 worst = worst_of(worst, r);
             }
         } else {
+            SPK_TRY(ensure_fp32(s));
             // FP32 work columns, then the FP64 reduced unknowns (a lent
             // workspace holds them after its column blocks)
             const size_t fbytes = (sizeof(float) * wcols * n + 255) / 256 * 256;

@@ -175,7 +175,7 @@ struct spk_system {
     spk::DBuf<char> work;
     spk::DBuf<unsigned long long> d_norms;
     double anorm = 0.0;
-    int ell_reach = -1;
+    int ell_reach = -1, ell_chunk = 0;  // ell_chunk: most slots of four tiles from a multiple of four on
     spk::DBuf<double> stage_b, stage_x;  // device copies of host b / x for spk_solve
     char *ext_ws = nullptr;  // caller-lent device workspace for the batched solves (spk_set_workspace)
     size_t ext_ws_bytes = 0;  // largest column distance from a tile's first row (-1: not computed)
@@ -272,6 +272,9 @@ int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool
 int chain_solve_host(spk_system *s, const double *b, double *x, double *db, double *dx);
 long long chain_device_check();
 int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *b, double *x, cudaStream_t st);
+bool residual_fits(const spk_system *s, int K);
+int residual_launch(const spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,
+                    long long ldr, unsigned long long *norms, cudaStream_t st);
 bool chain_rhs_one(spk_system *s, int fp32, int nk);
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
                     cudaStream_t st, int acc = 0);

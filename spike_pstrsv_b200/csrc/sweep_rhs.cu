@@ -296,7 +296,11 @@ __device__ bool solve_range(const RhsSweep &A, const Smem<T, NW * 8 * R, R> &M, 
             const double d = lds1(rd + 8 * (4 * k + q), 0.0);
             double b[R];
 #pragma unroll
-            for (int u = 0; u < R; u++) b[u] = lds1(st + boff + 17 * 8 * u + 32 * k, 0.0);
+            for (int u = 0; u < R; u++) {
+                b[u] = lds1(st + boff + 17 * 8 * u + 32 * k, 0.0);
+                // a right-hand side past FP32's range overflows in FP32, as the values would
+                if (sizeof(T) == 4) b[u] = fabs(b[u]) <= 3.4028234663852886e38 ? b[u] : b[u] * 1e308;
+            }
             T s[2][R];
 #pragma unroll
             for (int u = 0; u < R; u++) s[0][u] = s[1][u] = T(0);
