@@ -1353,7 +1353,11 @@ int chain_solve_host(spk_system *s, const double *b, double *x, double *db, doub
     }
     const int nch = (int)(s->ov_host.len ? s->ov_host.h1.size() : s->ov.len ? s->ov.h1.size()
                           : s->cp_host.len > 0 ? s->cp_host.h1.size() : s->h_ctasks1.size());
-    int K = 16;
+    // Chunks: each costs about 5 us of copies and events, and the copies overlap the more of
+    // them there are.  1 / 8 / 16 / 32 chunks: 16,384 rows 86 / 126 / 163 / 247 us, 524,288 rows
+    // 328 / 284 / 316 / 390 us, 1,048,576 rows 482 / 366 / 416 / 500 us, 4,194,304 rows
+    // 1,486 / 1,013 / 978 / 1,110 us.
+    int K = s->n < 65536 ? 1 : s->n < 2097152 ? 8 : 16;
     if (const char *e = getenv("SPK_PIPELINE_CHUNKS")) K = std::max(1, atoi(e));
     K = std::min(K, std::max(nch, 1));
     if (!s->st_in) {
