@@ -109,14 +109,15 @@ __global__ void __launch_bounds__(red_threads<K>()) k_reduced_csr(const RedArgs 
 //
 // Measured (one right-hand side, this kernel alone against one CTA on the CSR
 // copy): banded rows, 524,288 rows in 128 partitions, 126 levels of 61 rows: 690 ->
-// 221 us (1.75 us a level: the barrier and one row's dependent steps); band of 200,
-// 100,003 rows in 48 partitions, 46 levels of 176 rows: 958 -> 170 us; a 32^3
-// IC(0)-like factor in 8 partitions (CSR, levels of 1,024 rows): 925 -> 183 us.  32
-// systems of 1,024 to 131,072 rows, 364 columns: 20.3 -> 1.24 ms over the launches.
+// 218 us (1.7 us a level: the barrier's release waits 0.4 us for the remote stores, the rest
+// is one row's dependent steps; loading all of it two levels ahead changed nothing);
+// band of 200, 100,003 rows in 48 partitions, 46 levels of 176 rows: 958 -> 90 us (170 with
+// 8 warps a CTA, where some take two rows); a 32^3 IC(0)-like factor in 8 partitions (CSR,
+// levels of 1,024 rows): 925 -> 105 us (183).  32 systems of 1,024 to 131,072 rows, 364
+// columns: 20.3 -> 1.24 ms over the launches.
 template <int K>
 __host__ __device__ constexpr int ring_stride() { return K <= 2 ? K : K + 2; }  // doubles per unknown: 16-byte reads, no bank conflicts
-constexpr int kRingThreads = 256;
-constexpr int kRingWarps = kRingThreads / 32;
+constexpr int kRingWarps = 8;  // per CTA; 16 with one or two columns and more rows a level than 16 CTAs have warps
 constexpr size_t kRingBytes = 208 * 1024;
 
 struct RedLevel {  // rows rr[q0, q0 + nr); columns [c0, c0 + w); unknowns [f0, f1) enter with it; dense block at D + d
@@ -153,8 +154,8 @@ __device__ __forceinline__ void dsmem_store(unsigned local, unsigned cta, double
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote), "d"(v) : "memory");
 }
 
-template <int K, typename T, bool CSR>
-__global__ void __launch_bounds__(kRingThreads, 2) k_reduced_ring(const RingArgs *__restrict__ tab, RingArgs one) {
+template <int K, typename T, bool CSR, int TH>
+__global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const RingArgs *__restrict__ tab, RingArgs one) {
     constexpr int KS = ring_stride<K>(), RB = !CSR && K >= 4 ? 2 : 1;
     constexpr int LK = K == 8 ? 3 : (K == 4 ? 2 : (K == 2 ? 1 : 0));
     constexpr int PF = RB == 2 ? 4 : 8;                  // columns / 32 whose coefficients are loaded ahead
@@ -163,10 +164,10 @@ __global__ void __launch_bounds__(kRingThreads, 2) k_reduced_ring(const RingArgs
     const unsigned C = cluster_size(), rank = cluster_rank();
     const RingArgs A = tab ? tab[blockIdx.x / C] : one;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int gw = ((int)rank * kRingWarps + (tid >> 5)) * RB, nw = (int)C * kRingWarps * RB;
+    const int gw = ((int)rank * (TH / 32) + (tid >> 5)) * RB, nw = (int)C * (TH / 32) * RB;
     T *xb = (T *)A.xbuf + (long long)blockIdx.y * K * A.n;
     auto fill = [&](int lo, int hi) {
-        for (int id = lo + tid; id < hi; id += kRingThreads) {
+        for (int id = lo + tid; id < hi; id += TH) {
             const T *x = xb + A.mapRedX[id];
 #pragma unroll
             for (int k = 0; k < K; k++) ring[(id & A.mask) * KS + k] = (double)x[(long long)k * A.n];
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(kRingThreads, 2) k_reduced_ring(const RingArgs
         }
 #pragma unroll
         for (int u = 0; u < FU; u++) {
-            const int id = E.f0 + tid + kRingThreads * u;
+            const int id = E.f0 + tid + TH * u;
             fid[u] = id < E.f1 ? A.mapRedX[id] : -1;
         }
         if constexpr (CSR) {
@@ -332,12 +333,12 @@ __global__ void __launch_bounds__(kRingThreads, 2) k_reduced_ring(const RingArgs
 #pragma unroll
             for (int u = 0; u < FU; u++) {
                 if (fid[u] >= 0) {
-                    const int id = N.f0 + tid + kRingThreads * u;
+                    const int id = N.f0 + tid + TH * u;
 #pragma unroll
                     for (int k = 0; k < K; k++) ring[(id & A.mask) * KS + k] = fv[u][k];
                 }
             }
-            fill(N.f0 + kRingThreads * FU, N.f1);
+            fill(N.f0 + TH * FU, N.f1);
         }
         cluster_arrive();
         L = N;
@@ -407,19 +408,19 @@ RingArgs ring_args(const spk_system *s, void *work, int slots) {
 struct RingLaunch {
     const RingArgs *tab;
     RingArgs one;
-    int nsys, nblk, slots, ctas;
+    int nsys, nblk, slots, ctas, warps;
     cudaStream_t st;
     int *max_clusters;  // not null: query the clusters the device holds instead of launching
 };
 
-template <int K, typename T, bool CSR>
-int ring_go(const RingLaunch &R) {
-    auto kern = k_reduced_ring<K, T, CSR>;
+template <int K, typename T, bool CSR, int TH>
+int ring_go_t(const RingLaunch &R) {
+    auto kern = k_reduced_ring<K, T, CSR, TH>;
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingBytes));
     SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(R.nsys * R.ctas), (unsigned)R.nblk);
-    cfg.blockDim = dim3(kRingThreads);
+    cfg.blockDim = dim3(TH);
     cfg.dynamicSmemBytes = (size_t)R.slots * ring_stride<K>() * sizeof(double);
     cfg.stream = R.st;
     cudaLaunchAttribute at[1];
@@ -434,6 +435,13 @@ int ring_go(const RingLaunch &R) {
     }
     SPK_CUDA(cudaLaunchKernelEx(&cfg, kern, R.tab, R.one));
     return SPK_OK;
+}
+
+template <int K, typename T, bool CSR>
+int ring_go(const RingLaunch &R) {
+    if constexpr (K <= 2)
+        if (R.warps == 16) return ring_go_t<K, T, CSR, 512>(R);
+    return ring_go_t<K, T, CSR, 256>(R);
 }
 
 int ring_launch(int K, int fp32, bool csr, const RingLaunch &R) {
@@ -528,11 +536,12 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     if (c == 16) {
         const int k = ring_cols(need, 8);
         int fits = 0;
-        RingLaunch R{nullptr, ring_args(s, nullptr, 64), 1, 1, ring_slots(k, need), 16, st, &fits};
+        RingLaunch R{nullptr, ring_args(s, nullptr, 64), 1, 1, ring_slots(k, need), 16, kRingWarps, st, &fits};
         SPK_TRY(ring_launch(k, 0, !s->red_dense.p, R));
         if (fits < 1) c = 8;
     }
     s->red_ctas = c;
+    s->red_warps = avg > 16 * kRingWarps ? 16 : kRingWarps;
     s->red_ring = need;
     return SPK_OK;
 }
@@ -542,7 +551,7 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
 int reduced_solve(spk_system *s, int fp32, int ncols, void *work, cudaStream_t st) {
     if (s->red_ring) {
         const int k = ring_cols(s->red_ring, ncols), slots = ring_slots(k, s->red_ring);
-        const RingLaunch R{nullptr, ring_args(s, work, slots), 1, (ncols + k - 1) / k, slots, s->red_ctas, st, nullptr};
+        const RingLaunch R{nullptr, ring_args(s, work, slots), 1, (ncols + k - 1) / k, slots, s->red_ctas, s->red_warps, st, nullptr};
         SPK_TRY(ring_launch(k, fp32, !s->red_dense.p, R));
     } else {
         int K = 1;
@@ -569,6 +578,7 @@ int red_plan_build(RedPlan &p, const std::vector<RedMember> &members, int K, int
         ring[w].push_back(ring_args(m.s, m.work, slots));
         p.slots[w] = std::max(p.slots[w], slots);
         p.ctas[w] = std::max(p.ctas[w], m.s->red_ctas);
+        p.warps[w] = std::max(p.warps[w], m.s->red_warps);
     }
     auto put = [](DBuf<char> &d, const void *src, size_t bytes) -> int {
         if (!bytes) return SPK_OK;
@@ -601,7 +611,7 @@ int red_plan_launch(const RedPlan &p, cudaStream_t st, long long *kernels) {
     for (int w = 0; w < 8; w++) {
         if (!p.nring[w]) continue;
         const int k = 8 >> (w & 3);
-        const RingLaunch R{(const RingArgs *)p.ring[w].p, RingArgs{}, p.nring[w], p.K / k, p.slots[w], p.ctas[w], st,
+        const RingLaunch R{(const RingArgs *)p.ring[w].p, RingArgs{}, p.nring[w], p.K / k, p.slots[w], p.ctas[w], p.warps[w], st,
                            nullptr};
         SPK_TRY(ring_launch(k, p.fp32, w >= 4, R));
         ++*kernels;

@@ -16,7 +16,7 @@ struct RedMember {
 
 struct RedPlan {
     DBuf<char> csr, ring[8];  // argument tables: the one-CTA solve; clusters, by column block and layout
-    int ncsr = 0, nring[8] = {}, slots[8] = {}, ctas[8] = {};
+    int ncsr = 0, nring[8] = {}, slots[8] = {}, ctas[8] = {}, warps[8] = {};
     int K = 0, fp32 = 0;
 };
 

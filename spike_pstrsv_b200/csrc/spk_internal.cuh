@@ -234,7 +234,7 @@ struct spk_system {
     spk::DBuf<int4> d_red_rr;
     spk::DBuf<double> red_dense;
     int red_ring = 0;   // unknowns a level spans (0: the one-CTA solve on the CSR copy)
-    int red_ctas = 1;   // CTAs per cluster
+    int red_ctas = 1, red_warps = 8;  // CTAs per cluster, warps per CTA
     int dbg_fail_waits = 0;  // test hook: solve kernels report a failed wait at entry (spk_debug_set)
     int lean = 0;  // spk_compact: only what the chain solves read is kept (partition paths refused)
     double *red_scratch = nullptr;  // FP64 reduced unknowns of the FP32 batched solve in flight
