@@ -3,8 +3,8 @@ solve kernels.  Not part of the library: it drives the library the way a user
 would, so that a capture sees only the solve's own launches.
 
     python profile_case.py --m 2097152 --P 512 --nrhs 1
-        plain FP64 solves (spk_solve_device: k_chain_solve, or k_tile_solve with
-        --no-chain)
+        plain FP64 solves (spk_solve_device: k_sweep on tasks of the chain path, on
+        the partitions with --no-chain)
     python profile_case.py --m 2097152 --P 512 --nrhs 32 --mode 1
         batched solves (spk_solve_batch; FP32 + one refinement step with mode 1)
 
