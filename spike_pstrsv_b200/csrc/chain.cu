@@ -1137,6 +1137,12 @@ int chain_prepare(spk_system *s) {
         chain_release(s, true);
         return SPK_OK;
     }
+    if (s->sw_ok) {
+        SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
+        const long long lb = batch_overlap_rows(s, sms);
+        if (s->ov.len) SPK_TRY(build_overlap(s, lb, s->ov_batch));
+    }
+    if (s->ov_batch.len) return SPK_OK;
     // the batched kernel keeps fewer tasks resident (a wider window): its own
     // chains, as many as it keeps resident
     int occb = 4;
@@ -1145,11 +1151,6 @@ int chain_prepare(spk_system *s) {
     lenb = std::max<long long>(lenb, s->ch_len);
     if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) lenb = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     if (lenb > s->ch_len) SPK_TRY(build_plan(s, lenb, reach, &s->cp_batch));
-    if (s->sw_ok) {
-        SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
-        const long long lb = batch_overlap_rows(s, sms);
-        if (s->ov.len) SPK_TRY(build_overlap(s, lb, s->ov_batch));
-    }
     return SPK_OK;
 }
 
