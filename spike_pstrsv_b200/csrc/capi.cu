@@ -623,7 +623,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
     if (!strcmp(name, "chain_rows_phase1")) return s->ch_rows1;
     if (!strcmp(name, "chain_rows_phase4")) return s->ch_rows4;
     if (!strcmp(name, "chain_tasks_phase4")) return s->nctasks4;
-    if (!strcmp(name, "chain_batch_rows")) return s->ov_batch.len ? s->ov_batch.len : s->cp_batch.len ? s->cp_batch.len : s->ch_len;
+    if (!strcmp(name, "chain_batch_rows")) return s->ov_batch_rows ? s->ov_batch_rows : s->cp_batch.len ? s->cp_batch.len : s->ch_len;
     // wall microseconds of the last preprocessing, by part
     if (!strncmp(name, "prep_us_", 8)) {
         static const char *parts[5] = {"reference", "spikes", "tasks", "ell", "chains"};
@@ -632,7 +632,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
     }
     // spk_tune's knobs under their own names
     if (!strcmp(name, "rows")) return s->ov.len ? s->ov.len : s->ch_len;
-    if (!strcmp(name, "batch_rows")) return s->ov_batch.len ? s->ov_batch.len : s->cp_batch.len ? s->cp_batch.len : s->ch_len;
+    if (!strcmp(name, "batch_rows")) return s->ov_batch_rows ? s->ov_batch_rows : s->cp_batch.len ? s->cp_batch.len : s->ch_len;
     if (!strcmp(name, "stages")) return s->ch_stages;
     if (!strcmp(name, "batch_path")) return s->batch_path;
     if (!strcmp(name, "chain_host_rows")) return s->ov_host.len ? s->ov_host.len : s->ov.len ? s->ov.len : s->cp_host.len ? s->cp_host.len : s->ch_len;

@@ -165,6 +165,25 @@ __global__ void k_chain_fill(int n, int ntiles, const int *__restrict__ ia, cons
     }
 }
 
+// cp.async (sm_80+): per-thread asynchronous global -> shared copies, tracked
+// by commit groups (no register scoreboard, so a tile in flight never stalls
+// the tile being solved)
+__device__ __forceinline__ void cpa16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cpa8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cpa4(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // ---- spikes of the chains -------------------------------------------------------------
 //
 // One warp per chain [a, q); lane owns spike columns lane + 32 cc (cc < C), i.e.
@@ -174,6 +193,11 @@ __global__ void k_chain_fill(int n, int ntiles, const int *__restrict__ ia, cons
 // X_r = -sum_k v'(r, r + off_k) X_{r + off_k}.  Each lane reads only its own
 // columns, so the ring needs no barrier.  f = the smallest row whose absolute
 // row sum exceeds tau (q when none).
+//
+// A row is one serial step, bound by latency: each 32-row tile comes by cp.async one tile
+// ahead (loads from global memory a row took more than the row's arithmetic), and the row
+// sums are taken eight rows at a time from a table of the lanes' shares (a shuffle tree a
+// row held up the next row).
 
 struct SpikeArgs {
     const int2 *chains;  // [a, q)
@@ -182,18 +206,40 @@ struct SpikeArgs {
     const unsigned *off;  // offset bytes as 32-bit words
     const int *ptr;
     int reach;
+    int stage;  // bytes of a staged tile (the widest: values, then offsets)
     double tau;
     int *first;
     long long nval, nptr;  // element counts (bounds of the checked build)
 };
 
+constexpr int kSumRows = 8, kSumPitch = 33;
+
+__host__ __device__ inline int spike_ring_bytes(int reach, int C) { return 8 * (reach + 1) * 32 * C; }
+
+inline int spike_smem_bytes(int reach, int C, int stage) {
+    return spike_ring_bytes(reach, C) + 2 * stage + 8 * kSumRows * kSumPitch;
+}
+
 template <int C>
 __global__ void __launch_bounds__(32) k_chain_spike(SpikeArgs A) {
-    extern __shared__ double ring[];  // [(reach + 1) * 32 * C]
+    extern __shared__ __align__(16) double ring[];  // [(reach + 1) * 32 * C], two stages, the lanes' sums
+    unsigned char *const stages = (unsigned char *)ring + spike_ring_bytes(A.reach, C);
+    double *const sums = (double *)(stages + 2 * A.stage);
     const int lane = threadIdx.x;
     const int2 ch = A.chains[blockIdx.x];
     const int a = ch.x, q = ch.y;
     const int R = A.reach + 1;
+    // tile j: values (256 bytes a slot), then offsets (32 bytes a slot); w is a multiple of four
+    auto stage_in = [&](int j, int p0, int w) {
+        unsigned char *dst = stages + (j & 1) * A.stage;
+        for (int i = lane; i < 16 * w; i += 32) cpa16(dst + 16 * i, A.val + CK(p0 + 2 * i, A.nval, 4));
+        for (int i = lane; i < 2 * w; i += 32)
+            cpa16(dst + 256 * w + 16 * i, A.off + CK((p0 >> 2) + 4 * i, A.nval / 4, 3));
+        cpa_commit();
+    };
+    const int jt = (q - 1) >> 5, jb = a >> 5;
+    int p0 = A.ptr[CK(jt, A.nptr, 1)], w = (A.ptr[CK(jt + 1, A.nptr, 2)] - p0) >> 5;
+    stage_in(jt, p0, w);
     // slot(q - 1) = 0, slot(q + j) = j + 1
     for (int s = 0; s < R; s++) {
 #pragma unroll
@@ -204,40 +250,65 @@ __global__ void __launch_bounds__(32) k_chain_spike(SpikeArgs A) {
     }
     int first = q;
     int sr = 0;  // slot of the current row
-    for (int r = q - 1; r >= a; r--) {
-        const int j = r >> 5, l = r & 31;
-        const int p0 = A.ptr[CK(j, A.nptr, 1)];
-        const int w = (A.ptr[CK(j + 1, A.nptr, 2)] - p0) >> 5;
-        double acc[C][2];
+    int pn = jt > jb ? A.ptr[CK(jt - 1, A.nptr, 1)] : 0;
+    for (int j = jt; j >= jb; j--) {
+        __syncwarp();  // the stage of tile j + 1 has been read
+        const int wn = (p0 - pn) >> 5;
+        if (j > jb) stage_in(j - 1, pn, wn);
+        else cpa_commit();
+        const int pnn = j - 1 > jb ? A.ptr[CK(j - 2, A.nptr, 1)] : 0;
+        cpa_wait<1>();
+        __syncwarp();
+        const double2 *val = (const double2 *)(stages + (j & 1) * A.stage);
+        const unsigned *off = (const unsigned *)((const unsigned char *)val + 256 * w);
+        const int r1 = min(q, 32 * j + 32) - 1, r0 = max(a, 32 * j);
+        for (int rt = r1; rt >= r0; rt -= kSumRows) {
+            const int rows = min(kSumRows, rt - r0 + 1);
+            for (int i = 0; i < rows; i++) {
+                const int l = (rt - i) & 31;
+                double acc[C][2];
 #pragma unroll
-        for (int cc = 0; cc < C; cc++) acc[cc][0] = acc[cc][1] = 0.0;
-        for (int k0 = 0; k0 < w; k0 += 4) {
-            const unsigned ow = __ldg(A.off + CK(((p0 + (k0 >> 2) * 128) >> 2) + l, A.nval / 4, 3));
-            const double2 va = __ldg((const double2 *)A.val + CK((p0 + (k0 >> 1) * 64) / 2 + l, A.nval / 2, 4));
-            const double2 vb = __ldg((const double2 *)A.val + CK((p0 + ((k0 >> 1) + 1) * 64) / 2 + l, A.nval / 2, 5));
-            const double v4[4] = {va.x, va.y, vb.x, vb.y};
+                for (int cc = 0; cc < C; cc++) acc[cc][0] = acc[cc][1] = 0.0;
+#pragma unroll 4
+                for (int g = 0; g < w >> 2; g++) {
+                    const unsigned ow = off[32 * g + l];
+                    const double2 va = val[64 * g + l], vb = val[64 * g + 32 + l];
+                    const double v4[4] = {va.x, va.y, vb.x, vb.y};
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int o = (ow >> (8 * u)) & 0xff;
-                int cs = sr + o;
-                cs -= cs >= R ? R : 0;
+                    for (int u = 0; u < 4; u++) {
+                        int cs = sr + (int)((ow >> (8 * u)) & 0xff);
+                        cs -= cs >= R ? R : 0;
 #pragma unroll
-                for (int cc = 0; cc < C; cc++)
-                    acc[cc][u & 1] = fma(-v4[u], ring[CK(cs * 32 * C + lane + 32 * cc, R * 32 * C, 6)], acc[cc][u & 1]);
+                        for (int cc = 0; cc < C; cc++)
+                            acc[cc][u & 1] =
+                                fma(-v4[u], ring[CK(cs * 32 * C + lane + 32 * cc, R * 32 * C, 6)], acc[cc][u & 1]);
+                    }
+                }
+                double s = 0.0;
+#pragma unroll
+                for (int cc = 0; cc < C; cc++) {
+                    const double x = acc[cc][0] + acc[cc][1];
+                    ring[CK(sr * 32 * C + lane + 32 * cc, R * 32 * C, 7)] = x;
+                    s += fabs(x);
+                }
+                sums[i * kSumPitch + lane] = s;
+                sr = sr == 0 ? R - 1 : sr - 1;
             }
-        }
-        double s = 0.0;
+            // lane 4 i + k adds a quarter of row rt - i
+            __syncwarp();
+            double s = 0.0;
+            if ((lane >> 2) < rows)
 #pragma unroll
-        for (int cc = 0; cc < C; cc++) {
-            const double x = acc[cc][0] + acc[cc][1];
-            ring[CK(sr * 32 * C + lane + 32 * cc, R * 32 * C, 7)] = x;
-            s += fabs(x);
+                for (int u = 0; u < 8; u++) s += sums[(lane >> 2) * kSumPitch + (lane & 3) + 4 * u];
+            s += __shfl_xor_sync(kFull, s, 1);
+            s += __shfl_xor_sync(kFull, s, 2);
+            const unsigned big = __ballot_sync(kFull, !(s <= A.tau));  // NaN counts as significant
+            if (big) first = rt - ((31 - __clz(big)) >> 2);
+            __syncwarp();
         }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (!(s <= A.tau)) first = r;  // NaN counts as significant
-        sr = sr == 0 ? R - 1 : sr - 1;
+        p0 = pn, w = wn, pn = pnn;
     }
+    cpa_wait<0>();
     if (lane == 0) A.first[blockIdx.x] = first;
 }
 
@@ -260,25 +331,6 @@ struct ChainArgs {
     int *err;
     int fail_entry;     // test hook: report a failed wait and return (spk_debug_set "fail_waits")
 };
-
-// cp.async (sm_80+): per-thread asynchronous global -> shared copies, tracked
-// by commit groups (no register scoreboard, so a tile in flight never stalls
-// the tile being solved)
-__device__ __forceinline__ void cpa16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cpa8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cpa4(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // tiles staged in shared memory per task: the one solved + NS - 1 in flight (NS is
 // a template parameter of the solve kernel, 2 or 3: s->ch_stages)
@@ -969,7 +1021,8 @@ int spike_firsts(spk_system *s, const std::vector<int2> &chains, std::vector<int
     A.nval = (long long)s->ch_val.n;
     A.nptr = (long long)s->ch_ptr.n;
     const int C = s->ch_reach <= 32 ? 1 : (s->ch_reach <= 64 ? 2 : 4);
-    const int smem = (int)sizeof(double) * (s->ch_reach + 1) * 32 * C;
+    A.stage = 288 * s->ch_sw;
+    const int smem = spike_smem_bytes(s->ch_reach, C, A.stage);
     switch (C) {
         case 1:
             SPK_TRY(allow_smem(k_chain_spike<1>));
@@ -1042,6 +1095,7 @@ void chain_release(spk_system *s, bool keep_overlap = false) {
         s->ov_host.release();
         s->ov_batch.release();
         s->ov_warm = 0;
+        s->ov_batch_rows = 0;
     }
     s->host_plan_tried = 0;
     if (s->pipe_exec) cudaGraphExecDestroy(s->pipe_exec);
@@ -1066,6 +1120,7 @@ long long overlap_rows(spk_system *s, int sms, int occ);
 long long overlap_warm(const spk_system *s);
 int build_overlap(spk_system *s, long long len, ChainPlan &out);
 long long batch_overlap_rows(const spk_system *s, int sms);
+int batch_chains(spk_system *s);
 
 // Build the chain layout, the chains' spikes and the two task lists; leaves
 // chain_ok = 0 (the partition-based solve) when truncation is off, the layout
@@ -1139,10 +1194,18 @@ int chain_prepare(spk_system *s) {
     }
     if (s->sw_ok) {
         SPK_TRY(build_overlap(s, overlap_rows(s, sms, occ), s->ov));
-        const long long lb = batch_overlap_rows(s, sms);
-        if (s->ov.len) SPK_TRY(build_overlap(s, lb, s->ov_batch));
+        // the batched solve's own plan: at its first call
+        if (s->ov.len) s->ov_batch_rows = (int)batch_overlap_rows(s, sms);
     }
-    if (s->ov_batch.len) return SPK_OK;
+    return s->ov_batch_rows ? SPK_OK : batch_chains(s);
+}
+
+// The two-phase plan of the batched kernel without 16-row records.
+int batch_chains(spk_system *s) {
+    const int n = s->n;
+    int dev = 0, sms = 148;
+    SPK_CUDA(cudaGetDevice(&dev));
+    SPK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // the batched kernel keeps fewer tasks resident (a wider window): its own
     // chains, as many as it keeps resident
     int occb = 4;
@@ -1150,7 +1213,7 @@ int chain_prepare(spk_system *s) {
     long long lenb = 32ll * ((n / (sms * (long long)std::max(occb, 1)) + 31) / 32);
     lenb = std::max<long long>(lenb, s->ch_len);
     if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) lenb = std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
-    if (lenb > s->ch_len) SPK_TRY(build_plan(s, lenb, reach, &s->cp_batch));
+    if (lenb > s->ch_len) SPK_TRY(build_plan(s, lenb, s->ch_reach, &s->cp_batch));
     return SPK_OK;
 }
 
@@ -1509,7 +1572,13 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
 // Whether nk right-hand sides go in one launch on 16-row records (made here on first use),
 // and may then be added to X.
 bool chain_rhs_one(spk_system *s, int fp32, int nk) {
-    if (!s->ov_batch.len || rhs_sweep_prepare(s, fp32) != SPK_OK) return false;
+    if (!s->ov_batch_rows) return false;
+    if (!s->ov_batch.len && (build_overlap(s, s->ov_batch_rows, s->ov_batch) != SPK_OK || !s->ov_batch.len)) {
+        s->ov_batch_rows = 0;  // two phases
+        batch_chains(s);
+        return false;
+    }
+    if (rhs_sweep_prepare(s, fp32) != SPK_OK) return false;
     return rhs_sweep_fits(s, fp32, nk);
 }
 
@@ -1638,7 +1707,7 @@ int chain_tune(spk_system *s, const char *name, long long v) {
         return SPK_ERR_ARG;
     }
     const long long len = 32ll * ((v + 31) / 32);
-    if (plain ? s->ov.len : s->ov_batch.len) {  // the one-launch solves take any length
+    if (plain ? s->ov.len : s->ov_batch_rows) {  // the one-launch solves take any length
         ChainPlan t;
         SPK_TRY(build_overlap(s, len, t));
         if (!t.len) {
@@ -1651,6 +1720,7 @@ int chain_tune(spk_system *s, const char *name, long long v) {
         to.d1.p = t.d1.p, to.d1.n = t.d1.n, t.d1.p = nullptr;
         to.h1.swap(t.h1);
         to.len = t.len;
+        if (!plain) s->ov_batch_rows = t.len;
         if (plain) {
             s->ov_host.release();
             s->host_plan_tried = 0;

@@ -2358,7 +2358,7 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
     const char *cb = getenv("SPK_CHAIN_BATCH");  // 1: always the chain kernels, 0: never
     const bool use_chain =
         s->chain_ok && (s->lean || (s->batch_path >= 0 ? s->batch_path == 1
-                                                       : (cb ? cb[0] == '1' : (mode == 0 || s->ov_batch.len || !part_wide))));
+                                                       : (cb ? cb[0] == '1' : (mode == 0 || s->ov_batch_rows || !part_wide))));
     if (!use_chain) SPK_TRY(partition_ensure(s));
     if (use_chain) {
         // the chain tasks fill the GPU whatever the partition count: every group

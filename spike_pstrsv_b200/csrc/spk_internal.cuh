@@ -193,7 +193,7 @@ struct spk_system {
     spk::ChainPlan cp_host;   // the host-array pipeline's chains (shorter; built on first use)
     // the one-launch solve on 16-row records: tasks that start ov_warm rows below their own
     spk::ChainPlan ov, ov_host, ov_batch;  // ov_batch: the batched solve's; ov_host: the host-array pipeline's, where ov's are too long
-    int ov_warm = 0;
+    int ov_warm = 0, ov_batch_rows = 0;  // ov_batch_rows: rows per task of ov_batch, which the first batched call builds
     int batch_path = -1;      // spk_tune "batch_path": 1 chain kernels, 0 partition kernels, -1 automatic
     // 16-row records of U for the one-right-hand-side solves (sweep.cu)
     int sw_ok = 0, sw_win = 0, sw_reach = 0, sw_wide = 0, sw_slots = 0, sw_stage = 0;
