@@ -28,6 +28,11 @@
 // * Solved rows stay in a window in shared memory that covers every column a row reaches,
 //   held twice, end to end, so that a column's address is one addition.  Rows from the
 //   task's top up come from `pre` (or are zero).
+// * An unused slot repeats its row's first column with value 0.  A row without any must not read
+//   one that it does not depend on (it may hold an infinity or a NaN, or, in `pre`, be one that
+//   phase 1 never writes): by a bit of the record its slots read a zero beside the window.  The
+//   choice is made on the address, a tile ahead: it costs nothing there (128 x 128 Poisson factor
+//   160 us, 176 us where the sum was dropped instead, on the way from one tile to the next).
 //
 // Measured (one solve, before -> after): banded rows with 16 off-diagonals, 4,194,304
 // rows: lower 234 -> 206 us (6 tasks an SM, 233 bytes a row: bound by HBM), its transpose
@@ -57,8 +62,10 @@ constexpr int kThreads = 64;        // a solving and a copying warp
 constexpr int kMaxSlots = 64;       // slots per lane
 constexpr int kMaxWindow = 8192;    // rows
 constexpr double kGrowth = 16.0;    // largest absolute row sum of W
-constexpr int kExtra = 1024 + 128;  // record: W, 1 / diagonal, then the number of extra slots,
-constexpr int kHead = kExtra + 16;  // then the slots' values and offsets, then the extra slots'
+// record: W, 1 / diagonal, then the number of extra slots (low 16 bits) and the rows that have a
+// column outside the tile (a bit each above them), the slots' values and offsets, the extra slots'
+constexpr int kExtra = 1024 + 128;
+constexpr int kHead = kExtra + 16;
 constexpr long long kWaitCycles = 1ll << 32;  // ~2 s: bound of a barrier wait
 constexpr int kCopyRows = 1024;     // rows per copy block
 constexpr int kMaxStages = 9;
@@ -92,11 +99,11 @@ __device__ __forceinline__ double lds(unsigned a) {
     return v;
 }
 
-// Shared memory of a task: full and empty barriers of the stages, the window, the stages.
+// Shared memory of a task: full and empty barriers of the stages, a zero, the window, the stages.
 struct Smem {
-    unsigned full, empty, win, stage0;
+    unsigned full, empty, zero, win, stage0;
     __device__ explicit Smem(unsigned base, int win_rows)
-        : full(base), empty(base + 8 * kMaxStages), win(base + 256), stage0(base + 256 + 16 * win_rows) {}
+        : full(base), empty(base + 8 * kMaxStages), zero(base + 16 * kMaxStages), win(base + 256), stage0(base + 256 + 16 * win_rows) {}
 };
 
 struct Ring {  // the stage a warp is at, and the parity of its next completion
@@ -153,6 +160,7 @@ struct Record {
     unsigned o[kWords], extra;
     double v[S], w[4], b, rd;
     __device__ __forceinline__ void load(unsigned st, unsigned lane, unsigned myrow, unsigned boff) {
+        extra = ldsu(st + kExtra);  // first: the tile's addresses wait for it
 #pragma unroll
         for (int h = 0; h < kWords; h++) o[h] = ldsu(st + kHead + 256 * S + 128 * h + 4 * lane);
 #pragma unroll
@@ -161,7 +169,6 @@ struct Record {
         rd = lds(st + 1024 + 8 * myrow);
 #pragma unroll
         for (int h = 0; h < 2; h++) lds2(st + 512 * h + 16 * lane, w[2 * h], w[2 * h + 1]);
-        extra = ldsu(st + kExtra);
     }
     __device__ __forceinline__ unsigned off(int u) const {
         return WIDE ? (u & 1 ? o[u / 2] >> 16 : o[u / 2] & 0xffffu) : (o[u / 4] >> (8 * (u & 3))) & 0xffu;
@@ -205,7 +212,9 @@ struct Solver {
     int src[4];         // lanes that hold r of this lane's columns in W
     bool isa2, isa3;    // whether its last two values belong to row g
     unsigned maskb, winb, boff;
+    unsigned outbit;    // of the record's word: the row has a column outside its tile
     unsigned pos;       // 8 * (first row of the tile above, modulo the window)
+    unsigned from;      // what the distances of the tile's outside columns count from
     int row, st_lo, st_hi;
     double *xp;
     int step;
@@ -227,6 +236,7 @@ struct Solver {
         maskb = 8u * (unsigned)(A.win - 1);
         winb = 8u * (unsigned)A.win;
         boff = A.stage - 128;
+        outbit = 0x10000u << myrow;
         const int jt = (hi - 1) >> 4;
         pos = (8u * (unsigned)(16 * jt + 16)) & maskb;
         row = 16 * jt + myrow;
@@ -236,10 +246,12 @@ struct Solver {
         step = A.rev_x ? 16 : -16;
     }
 
+    __device__ __forceinline__ unsigned base(const Record<S, WIDE> &C) const { return C.extra & outbit ? M.win + pos : M.zero; }
+
     // One tile: its record in C; the next one (if any) goes to N meanwhile.
     template <bool TOP>
     __device__ __forceinline__ bool tile(const Record<S, WIDE> &C, Record<S, WIDE> &N, bool more) {
-        const unsigned gather = M.win + pos, release = M.empty + 8 * R.slot, old = M.stage0 + R.slot * A.stage;
+        const unsigned gather = from, release = M.empty + 8 * R.slot, old = M.stage0 + R.slot * A.stage;
         double x[S];
 #pragma unroll
         for (int u = 0; u < S; u++) x[u] = lds(gather + 8 * C.off(u));
@@ -253,13 +265,15 @@ struct Solver {
 #pragma unroll
         for (int u = 0; u < S; u++) own[u & 1] = fma(C.v[u], x[u], own[u & 1]);
         double r = own[0] + own[1];
-        if (C.extra) r += extra_slots<WIDE>(old + kHead + slot_bytes(S, WIDE), C.extra, gather, lane);
+        if (C.extra & 0xffffu) r += extra_slots<WIDE>(old + kHead + slot_bytes(S, WIDE), C.extra & 0xffffu, gather, lane);
         r = fma(C.b, C.rd, -(r + __shfl_xor_sync(kFull, r, 1)));
         if (TOP && (row | 15) >= hi) {  // the task's top cuts the tile
             if (row >= hi) r = 0.0;
             else if (hi < A.n && A.pre) r = cut(A.ia, A.ja, A.a, row, hi, r, M.win, maskb);
             __syncwarp();
         }
+        pos = (pos - 128) & maskb;
+        from = base(N);  // here: N has arrived, and r is on its way
         const double r0 = __shfl_sync(kFull, r, src[0]), r1 = __shfl_sync(kFull, r, src[1]);
         const double r2 = __shfl_sync(kFull, r, src[2]), r3 = __shfl_sync(kFull, r, src[3]);
         double p0 = C.w[0] * r0, p1 = C.w[1] * r1;
@@ -270,7 +284,6 @@ struct Solver {
         double t = (second ? qa : pa) + __shfl_xor_sync(kFull, second ? pa : qa, 2);
         t += __shfl_xor_sync(kFull, t, 1);
         const double xv = r + t;  // one rounding at the size of x, as in the substitution
-        pos = (pos - 128) & maskb;
         const unsigned at = M.win + pos + 8 * myrow;
         if (!TOP || row < hi) {
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(xv) : "memory");
@@ -286,9 +299,11 @@ struct Solver {
 
     __device__ __forceinline__ bool run(int tiles) {
         Record<S, WIDE> P, Q;
+        Q.extra = 0;
         const unsigned bar = M.full + 8 * R.slot;
         if (!try_wait(bar, R.parity) && !slow_wait(bar, R.parity)) return false;
         P.load(M.stage0 + R.slot * A.stage, lane, myrow, boff);
+        from = base(P);
         if (!tile<true>(P, Q, tiles > 1)) return false;
         for (int k = 1; k < tiles; k += 2) {
             if (!tile<false>(Q, P, k + 1 < tiles)) return false;
@@ -341,6 +356,7 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(M.empty + 8 * k), "r"(1u) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("st.shared.f64 [%0], %1;" ::"r"(M.zero), "d"(0.0) : "memory");
     }
     __syncthreads();
     int lo, hi, st_lo, st_hi, skip_lo = 0, skip_hi = 0;
@@ -367,14 +383,12 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
         }
         return;
     }
-    // x of rows [r0, r0 + count) into the window (zero past the matrix or without pre); of what no
-    // row reads, the row after a cut tile is zeroed too: unused slots point there
+    // x of rows [r0, r0 + count) into the window (zero past the matrix or without pre)
     const unsigned maskb = 8u * (unsigned)(A.win - 1);
     auto load_window = [&](int r0, int count) {
-        for (int k = lane; k < max(A.reach, 17); k += 32) {
-            if (k >= count && k < A.reach) continue;
+        for (int k = lane; k < count; k += 32) {
             const int r = r0 + k;
-            const double v = A.pre && k < count && r < A.n ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
+            const double v = A.pre && r < A.n ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
             const unsigned at = M.win + ((8u * (unsigned)r) & maskb);
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + 8 * A.win), "d"(v) : "memory");
@@ -493,9 +507,10 @@ __global__ void __launch_bounds__(128) k_sweep_fill(int n, int ntiles, const int
         const double v = q < 15 - g ? W[g][g + 1 + q] : (q < 15 ? W[15 - g][q + 1] : 0.0);
         ((double *)R)[((u >> 1) * 32 + lane) * 2 + (u & 1)] = v;
     }
-    if (lane == 0) *(int4 *)(R + kExtra) = make_int4(E, 0, 0, 0);
-    // slot u of a lane: entry 2 u + (lane & 1) of its row's outside columns; unused slots
-    // repeat the row's first (or read the row after the tile) with value 0
+    const unsigned out = __ballot_sync(kFull, lane < 16 && e > f);
+    if (lane == 0) *(int4 *)(R + kExtra) = make_int4((int)((unsigned)E | out << 16), 0, 0, 0);
+    // slot u of a lane: entry 2 u + (lane & 1) of its row's outside columns; an unused one repeats
+    // the first (distance 0 where there is none: the zero)
     const int mine = (lane & 2) ? 15 - g : g;
     const int f0 = __shfl_sync(kFull, f, mine), n0 = __shfl_sync(kFull, e, mine) - f0;
     const double r0 = __shfl_sync(kFull, rd, mine);

@@ -57,8 +57,9 @@ template <typename T>
 __host__ __device__ constexpr int head_bytes() { return 160 * (int)sizeof(T) + 128; }  // W, 1 / diagonal (FP64)
 template <typename T>
 __host__ __device__ constexpr int base_bytes(int C) { return head_bytes<T>() + 64 * C * ((int)sizeof(T) + 4) + 16; }
-// base: W, 1 / diagonal, values [16][4 C], distances [16][4 C], number of extras (16 bytes);
-// then the extras, 16 bytes each: row, distance, value (FP64)
+// base: W, 1 / diagonal, values [16][4 C], distances [16][4 C], 16 bytes with the number of extras
+// and the rows that have a column outside the tile (a bit each; the others read a zero row beside
+// the window, not one they do not depend on); then the extras, 16 bytes each: row, distance, value (FP64)
 
 __device__ __forceinline__ unsigned su32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool try_wait(unsigned bar, unsigned parity) {
@@ -139,22 +140,22 @@ struct Ring {
     }
 };
 
-// Shared memory of a task: barriers, r of the tile, the window (win + mirror rows), the stages.
+// Shared memory of a task: barriers, r of the tile, a zero row, the window (win + mirror rows), the stages.
 // COLS columns padded to keep rows aligned for reads of R columns.
 template <typename T, int COLS, int R>
 struct Smem {
     static constexpr int LD = COLS + (R * (int)sizeof(T) >= 16 ? 16 / (int)sizeof(T) : R);
     unsigned full, empty;
-    T *r, *win;
+    T *r, *zero, *win;
     unsigned char *stage;
     __device__ Smem(unsigned char *base, int rows)
-        : full(su32(base)), empty(su32(base) + 8 * kMaxStages), r((T *)(base + 128)), win(r + 16 * LD),
+        : full(su32(base)), empty(su32(base) + 8 * kMaxStages), r((T *)(base + 128)), zero(r + 16 * LD), win(zero + LD),
           stage((unsigned char *)(((size_t)(win + (size_t)rows * LD) + 127) & ~(size_t)127)) {}
 };
 template <typename T>
 size_t smem_bytes(int cols, int per_lane, int rows, int ns, int stage) {
     const int ld = cols + (per_lane * (int)sizeof(T) >= 16 ? 16 / (int)sizeof(T) : per_lane);
-    return 128 + (size_t)(16 + rows) * ld * sizeof(T) + 128 + (size_t)ns * stage;
+    return 128 + (size_t)(17 + rows) * ld * sizeof(T) + 128 + (size_t)ns * stage;
 }
 
 // One task's walk over rows [lo, hi), as every warp of the block sees it.
@@ -273,21 +274,25 @@ __device__ bool solve_range(const RhsSweep &A, const Smem<T, NW * 8 * R, R> &M, 
         ring.next(A.ns);
         const unsigned rd = st + 160 * B, val = st + head_bytes<T>(), off = val + 64 * C * B;
         const int above = pos + 16 == A.win ? 0 : pos + 16;  // ring row of the tile above
-        const unsigned gat = wcol + above * LD;
+        const unsigned gat = wcol + above * LD, zero = rcol + 16 * LD;
         const bool top = 16 * j + 16 > g.hi, bottom = 16 * j < g.lo;
         T r[4][R];
         int4 o[C];
 #pragma unroll
         for (int e = 0; e < C; e++) o[e] = ldsi4(off + 16 * (C * q + e));
+        int ne, has;
+        asm volatile("ld.shared.v2.s32 {%0, %1}, [%2];" : "=r"(ne), "=r"(has) : "r"(st + base_bytes<T>(C) - 16) : "memory");
+        has >>= q;
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             T x[4 * C][R], v[4 * C];
+            const unsigned from = has >> 4 * k & 1 ? gat : zero;  // distances of a row without any are 0
 #pragma unroll
             for (int e = 0; e < C; e++) {
-                lds(gat + o[e].x * LD, x[4 * e]);
-                lds(gat + o[e].y * LD, x[4 * e + 1]);
-                lds(gat + o[e].z * LD, x[4 * e + 2]);
-                lds(gat + o[e].w * LD, x[4 * e + 3]);
+                lds(from + o[e].x * LD, x[4 * e]);
+                lds(from + o[e].y * LD, x[4 * e + 1]);
+                lds(from + o[e].z * LD, x[4 * e + 2]);
+                lds(from + o[e].w * LD, x[4 * e + 3]);
             }
             lds(val + 4 * C * B * (4 * k + q), v);
             if (k < 3)
@@ -326,8 +331,6 @@ __device__ bool solve_range(const RhsSweep &A, const Smem<T, NW * 8 * R, R> &M, 
         }
 #pragma unroll
         for (int k = 0; k < 4; k++) sts(rcol + (4 * k + q) * LD, r[k]);
-        int ne;
-        asm volatile("ld.shared.s32 %0, [%1];" : "=r"(ne) : "r"(st + base_bytes<T>(C) - 16) : "memory");
         if (ne) {
             __syncwarp();
             const unsigned ex = st + base_bytes<T>(C);
@@ -421,19 +424,18 @@ __device__ __forceinline__ void rhs_task(const RhsSweep &A, int task) {
     const int lo1 = two ? skip_hi : lo;  // first range [lo1, hi), second [lo, skip_lo)
     Ring R;
     bool ok = true;
-    // row r has ring row r modulo win; of what no row reads, the row after a cut tile is zeroed
-    // too: unused coefficients point there
+    // row r has ring row r modulo win
     auto load_window = [&](int r0, int count) {
         const T *pre = (const T *)A.pre;
-        const int p0 = r0 % A.win, rows = max(A.reach, 17);
-        for (int e = threadIdx.x; e < rows * COLS; e += NW * 32) {
-            const int k = e / rows, i = e - k * rows, r = r0 + i, p = p0 + i >= A.win ? p0 + i - A.win : p0 + i;
-            if (i >= count && i < A.reach) continue;
-            const T v = pre && i < count && r < A.n && k < A.nk ? pre[(long long)k * A.n + r] : T(0);
+        const int p0 = r0 % A.win;
+        for (int e = threadIdx.x; e < count * COLS; e += NW * 32) {
+            const int k = e / count, i = e - k * count, r = r0 + i, p = p0 + i >= A.win ? p0 + i - A.win : p0 + i;
+            const T v = pre && r < A.n && k < A.nk ? pre[(long long)k * A.n + r] : T(0);
             M.win[p * LD + k] = v;
             if (p < A.mirror) M.win[(p + A.win) * LD + k] = v;
         }
     };
+    if (threadIdx.x < COLS) M.zero[threadIdx.x] = T(0);
     for (int part = 0; part < (two ? 2 : 1); part++) {
         const Range g = part ? Range(lo, skip_lo) : Range(lo1, hi);
         // the second range reads the rows between, and above them those of the first
@@ -487,6 +489,8 @@ __device__ __forceinline__ void sw_slot(const unsigned char *R, int S, int E, in
     o = WIDE ? ((const unsigned short *)at)[((u >> 1) * 32 + lane) * 2 + (u & 1)] : at[((u >> 2) * 32 + lane) * 4 + (u & 3)];
 }
 
+__device__ __forceinline__ int extra_slots(const unsigned char *R) { return *(const int *)(R + 1152) & 0xffff; }
+
 __device__ __forceinline__ int lane_row(int lane) { return (lane & 2) ? 15 - (lane >> 2) : lane >> 2; }
 
 // Outside coefficients of this lane's row up to the last nonzero one.
@@ -509,7 +513,7 @@ __global__ void k_rhs_sizes(int nt, const int2 *__restrict__ sw_hdr, const unsig
     const int lane = threadIdx.x & 31, j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= nt) return;
     const unsigned char *R = sw_rec + (unsigned long long)(unsigned)sw_hdr[j].x * 16;
-    int e = max(0, row_count<WIDE>(R, S, *(const int *)(R + 1152), lane) - 4 * C);
+    int e = max(0, row_count<WIDE>(R, S, extra_slots(R), lane) - 4 * C);
     e = (lane & 1) ? 0 : e;
 #pragma unroll
     for (int o = 16; o; o >>= 1) e += __shfl_xor_sync(kFull, e, o);
@@ -532,7 +536,7 @@ __global__ void k_rhs_fill(int nt, const int2 *__restrict__ sw_hdr, const unsign
     const unsigned char *R = sw_rec + (unsigned long long)(unsigned)sw_hdr[j].x * 16;
     if (!extras && lane == 0) hdr[j] = make_int2((int)((unsigned)j * (base_bytes<T>(C) / 16)), base_bytes<T>(C));
     unsigned char *D = rec + (extras ? (unsigned long long)(unsigned)hdr[j].x : (unsigned long long)j * (base_bytes<T>(C) / 16)) * 16;
-    const int E = *(const int *)(R + 1152);
+    const int E = extra_slots(R);
     T *W = (T *)D, *val = (T *)(D + head_bytes<T>());
     int *off = (int *)(val + 64 * C);
     const double *Wf = (const double *)R;
@@ -560,7 +564,8 @@ __global__ void k_rhs_fill(int nt, const int2 *__restrict__ sw_hdr, const unsign
     const int total = __shfl_sync(kFull, before, 15);
     before -= ex;
     const int row = lane_row(lane), rc = __shfl_sync(kFull, c, row), rb = __shfl_sync(kFull, before, row);
-    if (lane == 0) *(int4 *)(D + base_bytes<T>(C) - 16) = make_int4(total, 0, 0, 0);
+    const unsigned out = __ballot_sync(kFull, lane < 16 && c > 0);
+    if (lane == 0) *(int4 *)(D + base_bytes<T>(C) - 16) = make_int4(total, (int)out, 0, 0);
     for (int at = lane; at < 64 * C; at += 32) {  // in the order of the record; unused places repeat the row's first column
         const int i = at / (4 * C), q = at - 4 * C * i, ci = __shfl_sync(kFull, c, i);
         const int l0 = i < 8 ? 4 * i : 4 * (15 - i) + 2;  // the first lane of row i
