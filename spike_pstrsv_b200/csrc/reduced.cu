@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(red_threads<K>()) k_reduced_csr(const RedArgs 
 // Coefficients are dense ([row][column] over the level's column range) when that
 // at most doubles the nonzeros: no column indices, and with four or more columns a
 // warp takes two rows, which halves the shared-memory reads of the unknowns (the
-// bound at eight columns).  Otherwise they stay in CSR order.
+// bound at eight columns).  A row whose sum is not finite is summed once more over its nonzeros,
+// so that an unknown reaches the rows that read it and no others.  Otherwise they stay in CSR order.
 //
 // Measured (one right-hand side, this kernel alone against one CTA on the CSR
 // copy): banded rows, 524,288 rows in 128 partitions, 126 levels of 61 rows: 690 ->
@@ -301,20 +302,45 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
             }
             // sums over the lanes: halves of the columns are exchanged while there are
             // several, so lane l ends with column l >> (5 - LK)
+            auto lane_sums = [&]() {
 #pragma unroll
-            for (int b = 0; b < RB; b++) {
+                for (int b = 0; b < RB; b++) {
 #pragma unroll
-                for (int s = 0; s < LK; s++) {
-                    const int h = K >> (s + 1), o = 16 >> s;
+                    for (int s = 0; s < LK; s++) {
+                        const int h = K >> (s + 1), o = 16 >> s;
 #pragma unroll
-                    for (int i = 0; i < h; i++) {
-                        const bool up = lane & o;
-                        const double give = up ? acc[b][i] : acc[b][i + h], keep = up ? acc[b][i + h] : acc[b][i];
-                        acc[b][i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                        for (int i = 0; i < h; i++) {
+                            const bool up = lane & o;
+                            const double give = up ? acc[b][i] : acc[b][i + h], keep = up ? acc[b][i + h] : acc[b][i];
+                            acc[b][i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                        }
                     }
-                }
 #pragma unroll
-                for (int o = 16 >> LK; o; o >>= 1) acc[b][0] += __shfl_xor_sync(0xffffffffu, acc[b][0], o);
+                    for (int o = 16 >> LK; o; o >>= 1) acc[b][0] += __shfl_xor_sync(0xffffffffu, acc[b][0], o);
+                }
+            };
+            lane_sums();
+            if constexpr (!CSR) {
+                bool odd = false;  // an infinity or a NaN, which a coefficient 0 may have let in: once more without those
+#pragma unroll
+                for (int b = 0; b < RB; b++) odd |= !(fabs(acc[b][0]) <= 1.7976931348623157e308);
+                if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+                    for (int b = 0; b < RB; b++) {
+#pragma unroll
+                        for (int k = 0; k < K; k++) acc[b][k] = 0.0;
+                        const double *d = A.D + L.d + (long long)min(q + b, L.nr - 1) * L.w;
+#pragma unroll 1
+                        for (int c = lane; c < L.w; c += 32) {
+                            const double v = d[c], *x = ring + ((L.c0 + c) & A.mask) * KS;
+                            if (v != 0.0)
+#pragma unroll
+                                for (int k = 0; k < K; k++) acc[b][k] = fma(v, x[k], acc[b][k]);
+                        }
+                        __syncwarp();
+                    }
+                    lane_sums();
+                }
             }
             const int k = lane >> (5 - LK), sub = lane & ((32 >> LK) - 1);
 #pragma unroll
