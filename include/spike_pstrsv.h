@@ -142,6 +142,8 @@ int spk_preproc(spk_system *s, const double *a, const int *ia, const int *ja, in
 
 /* Solve with device pointers b (n doubles, not modified) and x (n doubles) on
  * `stream` (a cudaStream_t passed as void*; NULL = the legacy default stream).
+ * x may be b itself (here, in spk_solve and in FP64 batches: column k of X in
+ * place of column k of B): such a solve takes the two-phase or partition kernels.
  * Asynchronous with respect to the host. */
 int spk_solve_device(spk_system *s, const double *b, double *x, void *stream);
 

@@ -30,7 +30,9 @@
 // the same values there as phase 4 would read.  The rows walked are those of both
 // phases plus `reach` a task, but the tasks need no other task's rows: their number
 // is free, down to 32 rows, and the walk's length is a + ov_warm instead of at least
-// twice the decay length.  262,147 rows, transpose: 80 -> 48 us; 5,003 rows: 47 -> 27 us.
+// twice the decay length.  They read b of rows that other tasks store: an x in b's place
+// takes the two phases, whose tasks read b of their own rows only (phase 4 of rows that
+// phase 1 has not stored).  262,147 rows, transpose: 80 -> 48 us; 5,003 rows: 47 -> 27 us.
 // spk_chain_phase keeps the two phases (a shard's rows end where another GPU's start).
 //
 // Kernel (systems without records, and the phases' layout).  One warp per task, lane = row of
@@ -1570,9 +1572,9 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
 }
 
 // Whether nk right-hand sides go in one launch on 16-row records (made here on first use),
-// and may then be added to X.
-bool chain_rhs_one(spk_system *s, int fp32, int nk) {
-    if (!s->ov_batch_rows) return false;
+// and may then be added to X.  apart: columns_apart(B, X).
+bool chain_rhs_one(spk_system *s, int fp32, int nk, bool apart) {
+    if (!s->ov_batch_rows || !apart) return false;
     if (!s->ov_batch.len && (build_overlap(s, s->ov_batch_rows, s->ov_batch) != SPK_OK || !s->ov_batch.len)) {
         s->ov_batch_rows = 0;  // two phases
         batch_chains(s);
@@ -1586,12 +1588,12 @@ bool chain_rhs_one(spk_system *s, int fp32, int nk) {
 // phase 1 then phase 4 of the right-hand-side-parallel chain kernel, in T
 // (double, or float with the FP32 copy of the values).  X is FP64.
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st, int acc) {
+                    cudaStream_t st, bool apart, int acc) {
     if (nk < 1 || nk > 32) {
         set_error(SPK_ERR_ARG, "chain batch of %d columns (1..32)", nk);
         return SPK_ERR_ARG;
     }
-    if (chain_rhs_one(s, fp32, nk)) {
+    if (chain_rhs_one(s, fp32, nk, apart)) {
         RhsSweep A = rhs_sweep_args(s, fp32, nk);
         A.tasks = s->ov_batch.d1.p;
         A.ntasks = (int)s->ov_batch.h1.size();
@@ -1642,9 +1644,9 @@ long long chain_device_check() {
 #endif
 }
 
-// One solve through the chain path: one launch, or phase 1 then phase 4, on stream st.
-int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring) {
-    if (s->ov.len) {
+// One solve through the chain path: one launch (b and x apart), or phase 1 then phase 4, on stream st.
+int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring, bool apart) {
+    if (s->ov.len && apart) {
         SPK_TRY(launch_chain<false>(s, s->ov.d1.p, (int)s->ov.h1.size(), b, x, st));
         if (prof) {
             cudaEventRecord(s->ev[ring][1], st);

@@ -2179,12 +2179,28 @@ int scaled_residual(spk_system *s, int K, cudaStream_t st, double *out) {
 // diag and ||A|| for the residuals (read from the CSR, which spk_compact releases)
 int residual_prepare(spk_system *s) { return ensure_residual(s); }
 
+bool columns_apart(long long n, int nrhs, const double *B, long long ldb, const double *X, long long ldx) {
+    const uintptr_t b = (uintptr_t)B, x = (uintptr_t)X;
+    const uintptr_t wb = sizeof(double) * (uintptr_t)((nrhs - 1) * ldb + n), wx = sizeof(double) * (uintptr_t)((nrhs - 1) * ldx + n);
+    if (b + wb <= x || x + wx <= b) return true;
+    if (ldb != ldx) return false;
+    // column j of X starts d + (j - i) ld bytes after column i of B; the two differences nearest -d / ld
+    // (and one more) are the only ones that can bring them within a column's width
+    const long long d = (long long)(x - b), ld = (long long)sizeof(double) * ldb, w = (long long)sizeof(double) * n;
+    for (long long j = -1; j <= 1; j++) {
+        const long long k = d / ld + j, gap = d - k * ld;
+        if (k > -nrhs && k < nrhs && gap < w && gap > -w) return false;
+    }
+    return true;
+}
+
 int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph) {
     if (!s->built) {
         set_error(SPK_ERR_STATE, "no preprocessed system");
         return SPK_ERR_STATE;
     }
-    const bool chains = (s->chain_ok || s->ov.len) && (!ph || s->lean);
+    const bool apart = columns_apart(s->n, 1, b, s->n, x, s->n);
+    const bool chains = (s->chain_ok || (s->ov.len && apart)) && (!ph || s->lean);
     if (!chains) SPK_TRY(partition_ensure(s));  // the partition path below
     double t0 = 0;
     auto lap = [&](int slot) {
@@ -2203,7 +2219,7 @@ int solve(spk_system *s, const double *b, double *x, cudaStream_t st, double *ph
         cudaEventRecord(s->ev[ring][0], st);
     }
     if (chains) {  // a compacted system has no other path (no phase times)
-        SPK_TRY(chain_solve(s, b, x, st, prof, ring));
+        SPK_TRY(chain_solve(s, b, x, st, prof, ring, apart));
     } else if ((s->ell_ok || s->sw_ok) && !ph) {
         SPK_TRY((launch_tiles<1, double>(s, b, s->n, x, s->n, s->xbuf.p, st, prof, ring)));
     } else {
@@ -2364,12 +2380,13 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
         // the chain tasks fill the GPU whatever the partition count: every group
         // of up to 32 columns is one right-hand-side-parallel chain solve (used
         // when the partitions alone give too few tasks to fill the GPU)
+        const bool apart = columns_apart(n, nrhs, B, ldb, X, ldx);
         for (int g = 0; g < nrhs;) {
             const int K = std::min(nrhs - g, 32);
             const double *Bg = B + g * ldb;
             double *Xg = X + g * ldx;
             if (mode == 0) {
-                SPK_TRY(chain_solve_rhs(s, 0, K, Bg, ldb, Xg, ldx, st));
+                SPK_TRY(chain_solve_rhs(s, 0, K, Bg, ldb, Xg, ldx, st, apart));
                 if (resid) {
                     SPK_TRY(residual(s, K, Xg, ldx, Bg, ldb, rbuf_p, n, st, true));
                     double r = 0;
@@ -2377,7 +2394,7 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                     worst = worst_of(worst, r);
                 }
             } else {
-                SPK_TRY(chain_solve_rhs(s, 1, K, Bg, ldb, Xg, ldx, st));
+                SPK_TRY(chain_solve_rhs(s, 1, K, Bg, ldb, Xg, ldx, st, apart));
                 int it = 0;
                 double r = -1.0;
                 for (;; it++) {
@@ -2389,11 +2406,11 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                         if ((tol >= 0 && r <= tol) || it == maxit) break;
                     }
                     if (it == maxit) break;
-                    if (chain_rhs_one(s, 1, K)) {
-                        SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, Xg, ldx, st, 1));
+                    if (chain_rhs_one(s, 1, K, true)) {
+                        SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, Xg, ldx, st, true, 1));
                         continue;
                     }
-                    SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, dbuf_p, n, st));
+                    SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, dbuf_p, n, st, true));
                     k_axpy<<<dim3(148, K), 256, 0, st>>>(s->n, K, dbuf_p, Xg, ldx);
                     SPK_CUDA(cudaGetLastError());
                 }

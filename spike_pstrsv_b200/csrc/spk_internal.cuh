@@ -268,19 +268,24 @@ int residual_prepare(spk_system *s);
 int chain_prepare(spk_system *s);
 int chain_tune(spk_system *s, const char *name, long long v);
 int partition_ensure(spk_system *s);
-int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring);
+int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring, bool apart);
 int chain_solve_host(spk_system *s, const double *b, double *x, double *db, double *dx);
 long long chain_device_check();
 int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *b, double *x, cudaStream_t st);
 bool residual_fits(const spk_system *s, int K);
 int residual_launch(const spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,
                     long long ldr, unsigned long long *norms, cudaStream_t st);
-bool chain_rhs_one(spk_system *s, int fp32, int nk);
+bool chain_rhs_one(spk_system *s, int fp32, int nk, bool apart);
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st, int acc = 0);
+                    cudaStream_t st, bool apart, int acc = 0);
 int check_device_error(spk_system *s);
 int collect_phase_times(spk_system *s);
 int collect_event_set(spk_system *s, int k);
+
+// Whether no column of B (nrhs columns of n rows, ldb apart) shares an element with one of X.  Tasks
+// of the one-launch solves read rows of b that other tasks store x of, so they need it; the two
+// phases and the partitions read a task's own rows only, before they are stored.
+bool columns_apart(long long n, int nrhs, const double *B, long long ldb, const double *X, long long ldx);
 
 // pointer classification
 int is_device_pointer(const void *p);
