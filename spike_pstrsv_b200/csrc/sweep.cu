@@ -41,9 +41,11 @@
 // Staged records: 2 / 3 / 4 / 6 a task take 180 / 99 / 80 / 80 us at 262,147 rows and 3 / 4 /
 // 5 / 6 take 233 / 211 / 208 / 194 us at full size.
 //
-// W is used only where its rows' absolute sums stay at most kGrowth: the error of the
-// product is then a small multiple of the substitution's own (c u |W||T||W||r| against
-// c u |W||T||x|).
+// W is used only where its rows' absolute sums stay at most kGrowth: the error of the product
+// grows with them (c u |W||T||W||r| against c u |W||T||x| of the substitution).  Over 40,000 random
+// triangles of 16 rows, against 80 bits, the product's mean error is 0.5 to 0.65 of the
+// substitution's for sums up to 4, 0.77 to 5.7, 0.98 to 8, 1.24 to 11 and 1.45 to 16, and its largest
+// one passes the substitution's from about 5 on: the limit is 4 (it was 16).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -61,7 +63,7 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 64;        // a solving and a copying warp
 constexpr int kMaxSlots = 64;       // slots per lane
 constexpr int kMaxWindow = 8192;    // rows
-constexpr double kGrowth = 16.0;    // largest absolute row sum of W
+constexpr double kGrowth = 4.0;     // largest absolute row sum of W
 // record: W, 1 / diagonal, then the number of extra slots (low 16 bits) and the rows that have a
 // column outside the tile (a bit each above them), the slots' values and offsets, the extra slots'
 constexpr int kExtra = 1024 + 128;
