@@ -322,7 +322,9 @@ int spk_compact(spk_system *s, long long *freed);
  * SPK_ERR_STATE unless spk_debug_scalar(s, "chain") == 1. */
 int spk_tune(spk_system *s, const char *name, long long value);
 
-/* Test hook (no reference counterpart): spk_debug_set(s, "fail_waits", 1) makes
+/* Test hooks (no reference counterpart): spk_debug_set(s, "fail_allocs", k) makes
+ * what a batch prepares on first use (its plan, its records) find no memory, k
+ * times; spk_debug_set(s, "fail_waits", 1) makes
  * every solve kernel of s report a failed bounded wait at entry, before it
  * issues any copy, until the failure has been reported once (SPK_ERR_TIMEOUT
  * from the synchronous solve or spk_check); the next solve then runs normally.

@@ -327,7 +327,8 @@ class System:
         return self
 
     def debug_set(self, name: str, value: int) -> "System":
-        """Test hooks (spk_debug_set): "fail_waits" makes the solve kernels report a
+        """Test hooks (spk_debug_set): "fail_allocs" makes what a batch prepares on first
+        use find no memory, so many times; "fail_waits" makes the solve kernels report a
         failed bounded wait until the failure has been reported once."""
         _check(lib().spk_debug_set(self.h, name.encode(), int(value)))
         return self

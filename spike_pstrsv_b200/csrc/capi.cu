@@ -684,6 +684,10 @@ int spk_debug_set(spk_system *s, const char *name, long long value) {
         set_error(SPK_ERR_ARG, "null argument");
         return SPK_ERR_ARG;
     }
+    if (!strcmp(name, "fail_allocs")) {
+        s->dbg_fail_allocs = (int)value;
+        return SPK_OK;
+    }
     if (!strcmp(name, "fail_waits")) {
         s->dbg_fail_waits = value != 0;
         return SPK_OK;

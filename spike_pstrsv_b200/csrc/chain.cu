@@ -1571,29 +1571,44 @@ int chain_pipeline(spk_system *s, const double *b, double *x, double *db, double
     return SPK_OK;
 }
 
-// Whether nk right-hand sides go in one launch on 16-row records (made here on first use),
-// and may then be added to X.  apart: columns_apart(B, X).
-bool chain_rhs_one(spk_system *s, int fp32, int nk, bool apart) {
-    if (!s->ov_batch_rows || !apart) return false;
-    if (!s->ov_batch.len && (build_overlap(s, s->ov_batch_rows, s->ov_batch) != SPK_OK || !s->ov_batch.len)) {
-        s->ov_batch_rows = 0;  // two phases
-        batch_chains(s);
-        return false;
-    }
-    if (rhs_sweep_prepare(s, fp32) != SPK_OK) return false;
-    return rhs_sweep_fits(s, fp32, nk);
+int debug_no_memory(spk_system *s) {
+    if (s->dbg_fail_allocs <= 0) return SPK_OK;
+    s->dbg_fail_allocs--;
+    set_error(SPK_ERR_NOMEM, "no memory (test hook)");
+    return SPK_ERR_NOMEM;
 }
 
-// Up to 32 right-hand sides (device, column-major) through the chain path: one launch, or
-// phase 1 then phase 4 of the right-hand-side-parallel chain kernel, in T
-// (double, or float with the FP32 copy of the values).  X is FP64.
+// Whether nk right-hand sides go in one launch on 16-row records (plan and records are made
+// here on first use), and may then be added to X.  apart: columns_apart(B, X).  No memory for
+// them is the caller's error, as for every first use; only a length that no start below makes
+// final leaves the two phases for good.
+int chain_rhs_one(spk_system *s, int fp32, int nk, bool apart, bool *one) {
+    *one = false;
+    if (!s->ov_batch_rows || !apart) return SPK_OK;
+    if (!s->ov_batch.len) {
+        SPK_TRY(debug_no_memory(s));
+        SPK_TRY(build_overlap(s, s->ov_batch_rows, s->ov_batch));
+        if (!s->ov_batch.len) {
+            SPK_TRY(batch_chains(s));
+            s->ov_batch_rows = 0;
+            return SPK_OK;
+        }
+    }
+    SPK_TRY(rhs_sweep_prepare(s, fp32));
+    *one = rhs_sweep_fits(s, fp32, nk);
+    return SPK_OK;
+}
+
+// Up to 32 right-hand sides (device, column-major) through the chain path: one launch
+// (chain_rhs_one), or phase 1 then phase 4 of the right-hand-side-parallel chain kernel, in
+// T (double, or float with the FP32 copy of the values).  X is FP64.  acc: added to X (one).
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st, bool apart, int acc) {
+                    cudaStream_t st, bool one, int acc) {
     if (nk < 1 || nk > 32) {
         set_error(SPK_ERR_ARG, "chain batch of %d columns (1..32)", nk);
         return SPK_ERR_ARG;
     }
-    if (chain_rhs_one(s, fp32, nk, apart)) {
+    if (one) {
         RhsSweep A = rhs_sweep_args(s, fp32, nk);
         A.tasks = s->ov_batch.d1.p;
         A.ntasks = (int)s->ov_batch.h1.size();
@@ -1606,6 +1621,10 @@ int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long 
         SPK_TRY(rhs_sweep_launch(s, A, fp32, st));
         s->launches++;
         return SPK_OK;
+    }
+    if (acc) {
+        set_error(SPK_ERR_STATE, "the two-phase chain batch does not add to X");
+        return SPK_ERR_STATE;
     }
     const ChainPlan &bp = s->cp_batch;
     const bool own = bp.len > 0;  // the batched kernel's own chains

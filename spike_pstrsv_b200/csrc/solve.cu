@@ -2385,8 +2385,10 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
             const int K = std::min(nrhs - g, 32);
             const double *Bg = B + g * ldb;
             double *Xg = X + g * ldx;
+            bool one = false;
+            SPK_TRY(chain_rhs_one(s, mode, K, apart, &one));
             if (mode == 0) {
-                SPK_TRY(chain_solve_rhs(s, 0, K, Bg, ldb, Xg, ldx, st, apart));
+                SPK_TRY(chain_solve_rhs(s, 0, K, Bg, ldb, Xg, ldx, st, one));
                 if (resid) {
                     SPK_TRY(residual(s, K, Xg, ldx, Bg, ldb, rbuf_p, n, st, true));
                     double r = 0;
@@ -2394,7 +2396,7 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                     worst = worst_of(worst, r);
                 }
             } else {
-                SPK_TRY(chain_solve_rhs(s, 1, K, Bg, ldb, Xg, ldx, st, apart));
+                SPK_TRY(chain_solve_rhs(s, 1, K, Bg, ldb, Xg, ldx, st, one));
                 int it = 0;
                 double r = -1.0;
                 for (;; it++) {
@@ -2406,11 +2408,11 @@ int solve_batch(spk_system *s, int nrhs, const double *B, long long ldb, double 
                         if ((tol >= 0 && r <= tol) || it == maxit) break;
                     }
                     if (it == maxit) break;
-                    if (chain_rhs_one(s, 1, K, true)) {
-                        SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, Xg, ldx, st, true, 1));
+                    if (one) {
+                        SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, Xg, ldx, st, one, 1));
                         continue;
                     }
-                    SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, dbuf_p, n, st, true));
+                    SPK_TRY(chain_solve_rhs(s, 1, K, rbuf_p, n, dbuf_p, n, st, one));
                     k_axpy<<<dim3(148, K), 256, 0, st>>>(s->n, K, dbuf_p, Xg, ldx);
                     SPK_CUDA(cudaGetLastError());
                 }

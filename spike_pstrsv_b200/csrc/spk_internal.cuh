@@ -76,6 +76,7 @@ struct DBuf {
                                   : cudaMalloc((void **)&p, count * sizeof(T));
         if (e != cudaSuccess) {
             p = nullptr;
+            cudaGetLastError();  // reported here; the next launch's check must not find it
             set_error(SPK_ERR_NOMEM, "cudaMalloc(%zu bytes) failed: %s", count * sizeof(T),
                       cudaGetErrorString(e));
             return SPK_ERR_NOMEM;
@@ -235,6 +236,7 @@ struct spk_system {
     spk::DBuf<double> red_dense;
     int red_ring = 0;   // unknowns a level spans (0: the one-CTA solve on the CSR copy)
     int red_ctas = 1, red_warps = 8;  // CTAs per cluster, warps per CTA
+    int dbg_fail_allocs = 0;  // test hook: what a batch makes on first use finds no memory, so many times (spk_debug_set)
     int dbg_fail_waits = 0;  // test hook: solve kernels report a failed wait at entry (spk_debug_set)
     int lean = 0;  // spk_compact: only what the chain solves read is kept (partition paths refused)
     double *red_scratch = nullptr;  // FP64 reduced unknowns of the FP32 batched solve in flight
@@ -275,9 +277,10 @@ int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *
 bool residual_fits(const spk_system *s, int K);
 int residual_launch(const spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,
                     long long ldr, unsigned long long *norms, cudaStream_t st);
-bool chain_rhs_one(spk_system *s, int fp32, int nk, bool apart);
+int debug_no_memory(spk_system *s);
+int chain_rhs_one(spk_system *s, int fp32, int nk, bool apart, bool *one);
 int chain_solve_rhs(spk_system *s, int fp32, int nk, const double *B, long long ldb, double *X, long long ldx,
-                    cudaStream_t st, bool apart, int acc = 0);
+                    cudaStream_t st, bool one, int acc = 0);
 int check_device_error(spk_system *s);
 int collect_phase_times(spk_system *s);
 int collect_event_set(spk_system *s, int k);

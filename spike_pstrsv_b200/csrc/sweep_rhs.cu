@@ -692,6 +692,7 @@ void rhs_sweep_choose(spk_system *s, const int *hist, int most) {
 
 int rhs_sweep_prepare(spk_system *s, int fp32) {
     if (s->rs_ok[fp32] || !s->sw_ok) return SPK_OK;
+    SPK_TRY(debug_no_memory(s));
     const int nt = (s->n + 15) / 16, S = s->sw_slots, C = s->rs_groups, blocks = (nt + 3) / 4;
     const int base = fp32 ? base_bytes<float>(C) : base_bytes<double>(C);
     cudaStream_t st = s->stream;
