@@ -1,5 +1,6 @@
 """Forms of the reduced solve: systems of two halves that do not read each other, one of
-them with a NaN in its right-hand side (a dense level holds both)."""
+them with a NaN in its right-hand side (a dense level holds both), and the one-CTA solve of
+systems whose levels span more unknowns than shared memory holds."""
 import numpy as np
 import pytest
 
@@ -7,6 +8,7 @@ import oracle
 import spike_pstrsv_b200 as spk
 from cases import rel_err
 from spike_pstrsv_b200 import synth
+from test_gpu_sweep import _with
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-12  # the repository's bound on x against the substitution
@@ -40,3 +42,47 @@ def test_a_nan_stays_in_its_half(k, mode):
     S.solve_batch(dB, dX, mode=mode, tol=-1.0, maxit=3, want_resid=False)
     X = dX.cpu().numpy()
     assert max(rel_err(x[~even], y[~even]) for x, y in zip(X, xs)) <= TOL
+
+
+@pytest.mark.parametrize("m,per_row,band,P", [(4003, 3, 8, 4), (20011, 16, 64, 40)])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("records", [True, False])
+def test_one_cta(m, per_row, band, P, uplo, records, monkeypatch):
+    """Forced, on either kind of phase kernels; FP64 and FP32 columns, powers of two and others."""
+    import torch
+
+    monkeypatch.setenv("SPK_DISABLE_RING", "1")
+    if not records:
+        monkeypatch.setenv("SPK_DISABLE_SWEEP", "1")
+    L = synth.banded_lower(m, per_row=per_row, band=band, seed=m)
+    A = L if uplo == "L" else synth.transpose(L)
+    S = spk.System().set_truncation(-1.0).preproc(A.a, A.ia, A.ja, m, P, uplo)
+    assert S.scalar("reduced_ring") == 0 and S.scalar("kept_reduced_rows") > 0
+    _, B = synth.make_rhs(A, seed=5, nrhs=32)
+    xs = np.stack([oracle.sequential_solve(A, b, uplo) for b in B])
+    assert rel_err(S.solve(B[0]), xs[0]) <= TOL
+    for k in (1, 2, 3, 4, 8, 13, 16, 31, 32):
+        dB = torch.from_numpy(B[:k]).cuda()
+        for mode in (0, 1):
+            dX = torch.zeros_like(dB)
+            S.solve_batch(dB, dX, mode=mode, tol=-1.0, maxit=3, want_resid=False)
+            assert max(rel_err(x, y) for x, y in zip(dX.cpu().numpy(), xs)) <= TOL, (k, mode)
+
+
+def test_levels_wider_than_shared_memory():
+    """300 partitions with 64 dependents each, and a row near the end that reads one near the
+    start: its level spans more unknowns than a column's ring (16,384) holds."""
+    import torch
+
+    m, P = 40011, 300
+    A = _with(m, [(m - 200, 5, 0.25)], synth.banded_lower(m, seed=3))
+    S = spk.System().set_truncation(-1.0).preproc(A.a, A.ia, A.ja, m, P, "L")
+    assert S.scalar("reduced_ring") == 0 and S.scalar("kept_reduced_rows") > 16384
+    _, B = synth.make_rhs(A, seed=8, nrhs=5)
+    xs = np.stack([oracle.sequential_solve(A, b, "L") for b in B])
+    assert rel_err(S.solve(B[0]), xs[0]) <= TOL
+    dB = torch.from_numpy(B).cuda()
+    for mode in (0, 1):
+        dX = torch.zeros_like(dB)
+        S.solve_batch(dB, dX, mode=mode, tol=-1.0, maxit=3, want_resid=False)
+        assert max(rel_err(x, y) for x, y in zip(dX.cpu().numpy(), xs)) <= TOL, mode
