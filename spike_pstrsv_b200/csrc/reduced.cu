@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(red_threads<K>()) k_reduced_csr(const RedArgs 
 // level after it.
 //
 // Coefficients are dense ([row][column] over the level's column range) when that
-// at most doubles the nonzeros: no column indices, and with four or more columns a
+// at most doubles the nonzeros of the kept rows: no column indices, and with four or more columns a
 // warp takes two rows, which halves the shared-memory reads of the unknowns (the
 // bound at eight columns).  A row whose sum is not finite is summed once more over its nonzeros,
 // so that an unknown reaches the rows that read it and no others.  Otherwise they stay in CSR order.
@@ -376,11 +376,12 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
     }
 }
 
-// First and last column of each level (columns are sorted in a row).
+// First and last column of each level (columns are sorted in a row), and the nonzeros of all.
 __global__ void k_red_span(int nkept, const int4 *__restrict__ rr, const int *__restrict__ level,
-                           const int *__restrict__ JT, int *__restrict__ cmin, int *__restrict__ cmax) {
+                           const int *__restrict__ JT, int *__restrict__ cmin, int *__restrict__ cmax, int *__restrict__ nnz) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nkept) return;
+    atomicAdd(nnz, rr[q].w - rr[q].z);
     atomicMin(&cmin[level[q]], JT[rr[q].z]);
     atomicMax(&cmax[level[q]], JT[rr[q].w - 1]);
 }
@@ -519,7 +520,8 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     const char *no = getenv("SPK_DISABLE_RING");  // test hook: the one-CTA solve
     if (!nk || (no && no[0] == '1')) return SPK_OK;
     cudaStream_t st = s->stream;
-    std::vector<int> level(nk), span(2 * nl, -1);
+    std::vector<int> level(nk), span(2 * nl + 1, -1);  // first and last columns, nonzeros of the kept rows
+    span[2 * nl] = 0;
     for (int li = 0; li < nl; li++) {
         span[li] = 2147483647;
         for (int q = off[li]; q < off[li + 1]; q++) level[q] = li;
@@ -529,9 +531,10 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     SPK_TRY(upload(d_span, span));
     SPK_TRY(s->d_red_rr.alloc(nk));
     k_red_rows<<<blocks_for(nk), 256, 0, st>>>(nk, s->d_red_rows.p, s->mapRedX.p, s->IT.p, s->d_red_rr.p);
-    k_red_span<<<blocks_for(nk), 256, 0, st>>>(nk, s->d_red_rr.p, d_level.p, s->JT.p, d_span.p, d_span.p + nl);
+    k_red_span<<<blocks_for(nk), 256, 0, st>>>(nk, s->d_red_rr.p, d_level.p, s->JT.p, d_span.p, d_span.p + nl,
+                                                  d_span.p + 2 * nl);
     SPK_CUDA(cudaGetLastError());
-    SPK_CUDA(cudaMemcpyAsync(span.data(), d_span.p, sizeof(int) * 2 * nl, cudaMemcpyDeviceToHost, st));
+    SPK_CUDA(cudaMemcpyAsync(span.data(), d_span.p, sizeof(int) * (2 * nl + 1), cudaMemcpyDeviceToHost, st));
     SPK_CUDA(cudaStreamSynchronize(st));
     std::vector<RedLevel> lv(nl);
     long long tot = 0;
@@ -549,7 +552,7 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     static_assert(sizeof(RedLevel) == 8 * sizeof(int), "levels are stored as eight ints");
     SPK_TRY(s->d_red_lv.alloc(8 * (size_t)nl));
     SPK_CUDA(cudaMemcpyAsync(s->d_red_lv.p, lv.data(), sizeof(RedLevel) * nl, cudaMemcpyHostToDevice, st));
-    if (tot <= 2 * s->nT) {
+    if (tot <= 2ll * span[2 * nl]) {
         SPK_TRY(s->red_dense.alloc(tot));
         SPK_CUDA(cudaMemsetAsync(s->red_dense.p, 0, sizeof(double) * tot, st));
         k_red_dense<<<(nk + 7) / 8, 256, 0, st>>>(nk, s->d_red_rr.p, d_level.p, s->JT.p, s->T.p,

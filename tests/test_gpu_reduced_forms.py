@@ -1,6 +1,7 @@
 """Forms of the reduced solve: systems of two halves that do not read each other, one of
 them with a NaN in its right-hand side (a dense level holds both), and the one-CTA solve of
-systems whose levels span more unknowns than shared memory holds."""
+systems whose levels span more unknowns than shared memory holds; levels whose kept rows
+are mostly zeros while the dropped ones are full."""
 import numpy as np
 import pytest
 
@@ -86,3 +87,43 @@ def test_levels_wider_than_shared_memory():
         dX = torch.zeros_like(dB)
         S.solve_batch(dB, dX, mode=mode, tol=-1.0, maxit=3, want_resid=False)
         assert max(rel_err(x, y) for x, y in zip(dX.cpu().numpy(), xs)) <= TOL, mode
+
+
+def _sparse_kept_full_dropped(m, block):
+    """Upper CSR, blocks of 256 rows.  Even rows of the first 64 read their own place a block up
+    (one column each, 1/2); odd ones read a chain through the rest of the block that ends in every
+    odd row of the next (32 columns each, 1/4 a step: below 2^-60 after 30)."""
+    ia, ja, a = [0], [], []
+    for r in range(m):
+        o, up = r % block, r - r % block + block
+        if o < 64 and o % 2 == 0:
+            cols, v = [r + block], 0.5
+        elif o < 64:
+            cols, v = [up - block + 64], 0.25
+        elif o < block - 1:
+            cols, v = [r + 1], 0.25
+        else:
+            cols, v = list(range(up + 1, up + 64, 2)), 0.25 / 32
+        cols = [c for c in cols if c < m]
+        ja += [r] + cols
+        a += [1.0] + [v] * len(cols)
+        ia.append(len(ja))
+    return synth.CSR(m, np.array(ia, np.int32), np.array(ja, np.int32), np.array(a))
+
+
+@pytest.mark.parametrize("k", [1, 8])
+def test_dropped_rows_do_not_make_a_level_dense(k):
+    import torch
+
+    m, block = 2560, 256
+    A = _sparse_kept_full_dropped(m, block)
+    S = spk.System().preproc(A.a, A.ia, A.ja, m, m // block, "U")
+    # 32 kept rows a level of one nonzero each, over 63 columns; the dropped ones have 32 each
+    assert S.scalar("chain") == 0 and S.scalar("reduced_ring") > 0
+    assert 0 < S.scalar("kept_reduced_rows") <= 32 * (m // block - 2)
+    assert S.scalar("reduced_dense") == 0
+    _, B = synth.make_rhs(A, seed=12, nrhs=k)
+    dB = torch.from_numpy(B).cuda()
+    dX = torch.zeros_like(dB)
+    S.solve_batch(dB, dX, mode=0, tol=-1.0, maxit=0, want_resid=False)
+    assert max(rel_err(x, oracle.sequential_solve(A, b, "U")) for x, b in zip(dX.cpu().numpy(), B)) <= TOL
