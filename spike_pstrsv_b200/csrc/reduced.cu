@@ -7,7 +7,10 @@
 // value, and no arithmetic touches them.  All arithmetic is FP64; FP32 work
 // columns are rounded once, when an unknown is stored back.
 #include <algorithm>
+#include <array>
 #include <cstdlib>
+#include <map>
+#include <mutex>
 
 #include "reduced.cuh"
 
@@ -486,6 +489,33 @@ int ring_launch(int K, int fp32, bool csr, const RingLaunch &R) {
     }
 }
 
+// The CTAs a cluster of this very launch may have: `want`, halved until the device can place one
+// such cluster.  Up to 8 CTAs are portable; 16 need a partition of the chip with room for as
+// many of the kernel's CTAs at this size (asked once per device and configuration).
+int ring_ctas(int K, int fp32, bool csr, int want, int warps, int slots, int *ctas) {
+    *ctas = want;
+    if (want <= 8) return SPK_OK;
+    static std::mutex mu;
+    static std::map<std::array<int, 7>, int> known;
+    int dev = 0;
+    SPK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(mu);
+    const std::array<int, 7> key{dev, K, fp32, csr, want, K <= 2 ? warps : kRingWarps, slots};
+    const auto at = known.find(key);
+    if (at != known.end()) {
+        *ctas = at->second;
+        return SPK_OK;
+    }
+    for (; *ctas > 8; *ctas >>= 1) {
+        int fits = 0;
+        const RingLaunch R{nullptr, RingArgs{}, 1, 1, slots, *ctas, warps, nullptr, &fits};
+        SPK_TRY(ring_launch(K, fp32, csr, R));
+        if (fits > 0) break;
+    }
+    known[key] = *ctas;
+    return SPK_OK;
+}
+
 template <typename T>
 int csr_go(int K, const RedArgs *tab, const RedArgs &one, int nsys, cudaStream_t st) {
     switch (K) {
@@ -560,17 +590,10 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
         SPK_CUDA(cudaGetLastError());
     }
     SPK_CUDA(cudaStreamSynchronize(st));
-    // a warp per row of an average level, at most 16 CTAs (8 where the device cannot place 16 together)
+    // a warp per row of an average level, at most 16 CTAs (fewer where a launch cannot place them: ring_ctas)
     const int avg = (nk + nl - 1) / nl;
     int c = 1;
     while (c < 16 && c * kRingWarps < avg) c <<= 1;
-    if (c == 16) {
-        const int k = ring_cols(need, 8);
-        int fits = 0;
-        RingLaunch R{nullptr, ring_args(s, nullptr, 64), 1, 1, ring_slots(k, need), 16, kRingWarps, st, &fits};
-        SPK_TRY(ring_launch(k, 0, !s->red_dense.p, R));
-        if (fits < 1) c = 8;
-    }
     s->red_ctas = c;
     s->red_warps = avg > 16 * kRingWarps ? 16 : kRingWarps;
     s->red_ring = need;
@@ -582,7 +605,9 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
 int reduced_solve(spk_system *s, int fp32, int ncols, void *work, cudaStream_t st) {
     if (s->red_ring) {
         const int k = ring_cols(s->red_ring, ncols), slots = ring_slots(k, s->red_ring);
-        const RingLaunch R{nullptr, ring_args(s, work, slots), 1, (ncols + k - 1) / k, slots, s->red_ctas, s->red_warps, st, nullptr};
+        int ctas = 0;
+        SPK_TRY(ring_ctas(k, fp32, !s->red_dense.p, s->red_ctas, s->red_warps, slots, &ctas));
+        const RingLaunch R{nullptr, ring_args(s, work, slots), 1, (ncols + k - 1) / k, slots, ctas, s->red_warps, st, nullptr};
         SPK_TRY(ring_launch(k, fp32, !s->red_dense.p, R));
     } else {
         int K = 1;
@@ -628,6 +653,7 @@ int red_plan_build(RedPlan &p, const std::vector<RedMember> &members, int K, int
         // smaller clusters rather than a second wave (two CTAs per SM)
         const int nb = K / (8 >> (w & 3));
         while (p.ctas[w] > 4 && (long long)p.ctas[w] * p.nring[w] * nb > 2ll * sms) p.ctas[w] >>= 1;
+        if (p.nring[w]) SPK_TRY(ring_ctas(8 >> (w & 3), fp32, w >= 4, p.ctas[w], p.warps[w], p.slots[w], &p.ctas[w]));
     }
     return SPK_OK;
 }

@@ -8,7 +8,7 @@ import pytest
 import oracle
 import spike_pstrsv_b200 as spk
 from cases import rel_err
-from spike_pstrsv_b200 import synth
+from spike_pstrsv_b200 import group, synth
 from test_gpu_sweep import _with
 
 pytestmark = pytest.mark.gpu
@@ -127,3 +127,24 @@ def test_dropped_rows_do_not_make_a_level_dense(k):
     dX = torch.zeros_like(dB)
     S.solve_batch(dB, dX, mode=0, tol=-1.0, maxit=0, want_resid=False)
     assert max(rel_err(x, oracle.sequential_solve(A, b, "U")) for x, b in zip(dX.cpu().numpy(), B)) <= TOL
+
+
+@pytest.mark.parametrize("k", [1, 4])
+def test_group_of_small_and_large_rings(k):
+    """One launch for a member with many CTAs on a small ring and one with a ring that fills shared memory."""
+    import torch
+
+    mats = [(synth.banded_lower(20011, per_row=16, band=250, seed=1), 30),
+            (synth.banded_lower(9001, per_row=60, band=1500, seed=2), 4)]
+    systems = [spk.System().set_truncation(-1.0).preproc(A.a, A.ia, A.ja, A.m, P, "L") for A, P in mats]
+    assert 256 < systems[0].scalar("reduced_ring") < 1024 and systems[1].scalar("reduced_ring") > 2048
+    rhs = [synth.make_rhs(A, seed=3, nrhs=k)[1] for A, _ in mats]
+    B = [torch.from_numpy(b).cuda() for b in rhs]
+    X = [torch.zeros_like(b) for b in B]
+    st = torch.cuda.Stream()
+    g = group.Group(systems, B, X, mode=0, iters=0, stream=st.cuda_stream)
+    g.solve()
+    st.synchronize()
+    for (A, _), b, x in zip(mats, rhs, X):
+        assert max(rel_err(u, oracle.sequential_solve(A, v, "L")) for u, v in zip(x.cpu().numpy(), b)) <= TOL
+    g.close()
