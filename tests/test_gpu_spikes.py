@@ -1,0 +1,35 @@
+"""The chains' spikes: every chain's first significant row against scipy's triangular
+solves, over one, two and four warps a chain, the ring full and not, few and many slots a
+row, chains that end with the matrix."""
+import numpy as np
+import pytest
+
+import spike_pstrsv_b200 as spk
+from chain_ref import chain_plan, upper
+from spike_pstrsv_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("per_row,band", [(1, 1), (3, 7), (8, 31), (8, 32), (12, 33), (16, 64), (40, 64), (8, 65), (17, 127),
+                                          (30, 128), (63, 128)])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+def test_first_significant_rows(per_row, band, uplo):
+    m = 3 * 1024 + 77
+    L = synth.banded_lower(m, per_row=per_row, band=band, seed=per_row * 1000 + band)
+    a = L.a.copy()
+    a[L.ia[1:] - 1] *= 32  # spikes that decay within a chain also where rows are long
+    L = synth.CSR(m, L.ia, L.ja, a)
+    A = L if uplo == "L" else synth.transpose(L)
+    S = spk.System().preproc(A.a, A.ia, A.ja, m, 4, uplo)
+    if np.diff(A.ia).max() > 65:  # more than 64 off-diagonals in a row (a column of L): no chains
+        assert S.scalar("chain") == 0
+        return
+    assert S.scalar("chain") == 1
+    want, reach = chain_plan(upper(A, uplo)[0], S.scalar("chain_rows"))
+    assert S.scalar("chain_reach") == reach
+    got = S.array("chain_tasks1").reshape(-1, 4)
+    want = want.reshape(-1, 4)
+    assert np.array_equal(got[:, :3], want[:, :3])
+    # a row whose sum rounds to either side of 2^-60 would move f by one
+    assert np.abs(got[:, 3] - want[:, 3]).max() <= 1
