@@ -1159,6 +1159,7 @@ int chain_rhs_occupancy(spk_system *s, int *occ);
 int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra);
 long long overlap_rows(spk_system *s, int sms, int occ);
 long long overlap_warm(const spk_system *s);
+long long warm_rows(long long need);
 int build_overlap(spk_system *s, long long len, ChainPlan &out);
 long long batch_overlap_rows(const spk_system *s, int sms);
 int batch_chains(spk_system *s);
@@ -1291,31 +1292,42 @@ long long overlap_rows(spk_system *s, int sms, int occ) {
     return best;
 }
 
+// Whole tiles of rows for a start `need` rows below, as measured from few places: from the many
+// places of a plan of short tasks it is up to 1.5 % more (banded rows with 16 off-diagonals, 64
+// columns: 1,050 from 32 places, 1,064 from 287), and a start that falls short by a few rows costs
+// a walk.
+long long warm_rows(long long need) { return 32 * ((need + need / 64 + 31) / 32); }
+
 // The decay length of the plan's spikes, and the rows that a task's first row may read.
 long long overlap_warm(const spk_system *s) {
     if (s->ov_warm) return s->ov_warm;
     long long redo = 0;
     for (const ChainTask &t : s->h_ctasks1) redo = std::max<long long>(redo, t.hi - t.st_hi);
-    return 32ll * ((redo + s->ch_reach + 31) / 32);
+    return warm_rows(redo + s->ch_reach);
 }
 
-// Tasks of `len` rows for the one-launch solve: the start below each task is raised until
-// the spike of the rows walked before the task's own is negligible in the first `reach`
-// of them, for every task; left empty (two phases) if it does not become so.
+// Tasks of `len` rows for the one-launch solve: the start below each task is raised (to the decay
+// length that the walk shows, then by quarters) until the spike of the rows walked before the
+// task's own is negligible in the first `reach` of them, for every task; left empty (two phases)
+// if it does not become so.
 int build_overlap(spk_system *s, long long len, ChainPlan &out) {
     const int n = s->n;
     out.release();
     long long warm = overlap_warm(s);
-    for (int tries = 0; tries < 6; tries++, warm += 32 * (warm / 128 + 1)) {
+    for (int tries = 0; tries < 6; tries++) {
         std::vector<int2> segs;
         for (long long q = len; q + warm < n; q += len) segs.push_back(make_int2((int)q, (int)(q + warm)));
-        bool ok = true;
+        long long need = 0;  // the longest decay, and the rows that must hold it
         if (!segs.empty()) {
             std::vector<int> first;
             SPK_TRY(spike_firsts(s, segs, first));
-            for (size_t c = 0; c < segs.size() && ok; c++) ok = first[c] >= segs[c].x + s->ch_reach;
+            for (size_t c = 0; c < segs.size(); c++)
+                need = std::max<long long>(need, first[c] > segs[c].x ? segs[c].y - first[c] + s->ch_reach : n);
         }
-        if (!ok) continue;
+        if (need > warm) {
+            warm = tries < 2 && need < n ? std::max(warm + 32, warm_rows(need)) : warm + 32 * (warm / 128 + 1);
+            continue;
+        }
         for (long long a = 0; a < n; a += len) {
             const long long q = std::min<long long>(a + len, n);
             out.h1.push_back(ChainTask{(int)a, (int)std::min<long long>(q + warm, n), (int)a, (int)q});
@@ -1352,7 +1364,7 @@ int build_plan(spk_system *s, long long len, int reach, ChainPlan *extra) {
             int redo = 0;
             for (size_t c = 1; c < chains.size(); c++)
                 redo = first[c] > chains[c].x ? std::max(redo, chains[c].y - first[c]) : n;
-            if (!extra) s->ov_warm = redo + reach < n ? 32 * ((redo + reach + 31) / 32) : 0;
+            if (!extra) s->ov_warm = redo + reach < n ? (int)warm_rows(redo + reach) : 0;
             continue;
         }
         if (!extra) s->ov_warm = 0;
