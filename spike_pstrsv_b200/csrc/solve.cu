@@ -2998,14 +2998,7 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
         if (const int rc = partition_ensure(s); rc != SPK_OK) return fail(rc);
         if (mode == 1 || nrhs[i] > 1)
             if (const int rc = rhs_sweep_prepare(s, mode); rc != SPK_OK) return fail(rc);
-        if (mode == 1) {
-            int rc = ensure_fp32(s);
-            if (rc == SPK_OK) rc = ensure_residual(s);
-            if (rc != SPK_OK) return fail(rc);
-        } else if (!s->diag.p) {
-            const int rc = ensure_residual(s);
-            if (rc != SPK_OK) return fail(rc);
-        }
+        if (const int rc = ensure_residual(s); rc != SPK_OK) return fail(rc);
         t1[i].resize(s->ntasks1);
         t4[i].resize(s->ntasks2);
         if (s->ntasks1 && cudaMemcpy(t1[i].data(), s->d_tasks1.p, sizeof(SegTask) * s->ntasks1,
@@ -3036,7 +3029,10 @@ int spk_group_create(spk_group **out, int count, spk_system *const *systems, con
                 v.R = (double *)(intptr_t)pool_bytes;
                 pool_bytes += (kn * 8 + 255) / 256 * 256;
                 v.D = (double *)(intptr_t)pool_bytes;
-                pool_bytes += (kn * 8 + 255) / 256 * 256;
+                if (kind_of(s, K, mode).path == GroupKind::kTiles) {  // the others add their correction to X
+                    if (const int rc = ensure_fp32(s); rc != SPK_OK) return fail(rc);
+                    pool_bytes += (kn * 8 + 255) / 256 * 256;
+                }
                 v.red = (double *)(intptr_t)pool_bytes;
                 pool_bytes += ((long long)K * s->nRed * 8 + 255) / 256 * 256;
             }
