@@ -580,7 +580,7 @@ int spk_compact(spk_system *s, long long *freed) {
     s->red_dense.release();
     s->d_red_lv.release();
     s->d_red_rr.release();
-    s->red_ring = 0;
+    s->red_ring = s->red_full = 0;
     s->d_copies.release();
     s->lean = 1;
     if (freed) *freed = before - spk_debug_scalar(s, "device_bytes");
@@ -609,7 +609,7 @@ long long spk_debug_scalar(const spk_system *s, const char *name) {
     }
     if (!strcmp(name, "chain")) return s->chain_ok;
     if (!strcmp(name, "sweep")) return s->sw_ok;
-    if (!strcmp(name, "reduced_dense")) return s->red_dense.p ? (long long)s->red_dense.n : 0;  // coefficients of dense levels
+    if (!strcmp(name, "reduced_dense")) return s->red_full ? (long long)s->red_dense.n : 0;  // coefficients of dense levels
     if (!strcmp(name, "reduced_ring")) return s->red_ring;  // unknowns a level spans (0: the one-CTA solve)
     if (!strcmp(name, "lean")) return s->lean;
     if (!strcmp(name, "device_check")) return chain_device_check();  // checked builds only

@@ -1280,7 +1280,7 @@ long long batch_overlap_rows(const spk_system *s, int sms) {
 long long overlap_rows(spk_system *s, int sms, int occ) {
     if (const char *e = getenv("SPK_CHAIN_ROWS")) return std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     const long long n = s->n, warm = overlap_warm(s);
-    const double tile_ns = 270 + 12.0 * s->sw_slots, row_bytes = (double)s->sw_rec.n / n + 16;
+    const double tile_ns = 270 + 12.0 * s->sw_slots, row_bytes = (double)s->sw_bytes / n + 16;
     long long best = 0;
     double best_t = 0;
     for (int w = 1; w <= std::min(std::max(occ, 1), 6); w++) {

@@ -431,7 +431,7 @@ int ring_cols(int need, int ncols) {
 }
 
 RingArgs ring_args(const spk_system *s, void *work, int slots) {
-    const bool dense = s->red_dense.p != nullptr;
+    const bool dense = s->red_full;
     return RingArgs{(const RedLevel *)s->d_red_lv.p, s->nlvl, s->d_red_rr.p, s->mapRedX.p,
                     dense ? s->red_dense.p : s->T.p, s->JT.p, work, s->n, s->nRed, slots - 1};
 }
@@ -542,10 +542,18 @@ RedArgs csr_args(const spk_system *s, void *work, double *red) {
 // spans more unknowns than shared memory holds for one column.
 int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vector<int> &off,
                     const std::vector<int> &lvl_first) {
-    s->red_dense.release();
-    s->d_red_lv.release();
-    s->d_red_rr.release();
+    // the tables of a system preprocessed again take the last ones' memory, as its records do
     s->red_ring = 0;
+    s->red_full = 0;
+    struct Unused {
+        spk_system *s;
+        ~Unused() {
+            if (!s->red_full) s->red_dense.release();
+            if (s->red_ring) return;
+            s->d_red_lv.release();
+            s->d_red_rr.release();
+        }
+    } unused{s};
     const int nl = s->nlvl, nk = s->nkept;
     const char *no = getenv("SPK_DISABLE_RING");  // test hook: the one-CTA solve
     if (!nk || (no && no[0] == '1')) return SPK_OK;
@@ -559,7 +567,7 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     DBuf<int> d_level(st), d_span(st);
     SPK_TRY(upload(d_level, level));
     SPK_TRY(upload(d_span, span));
-    SPK_TRY(s->d_red_rr.alloc(nk));
+    SPK_TRY(s->d_red_rr.reserve(nk));
     k_red_rows<<<blocks_for(nk), 256, 0, st>>>(nk, s->d_red_rows.p, s->mapRedX.p, s->IT.p, s->d_red_rr.p);
     k_red_span<<<blocks_for(nk), 256, 0, st>>>(nk, s->d_red_rr.p, d_level.p, s->JT.p, d_span.p, d_span.p + nl,
                                                   d_span.p + 2 * nl);
@@ -580,10 +588,11 @@ int reduced_prepare(spk_system *s, const std::vector<int> &rows, const std::vect
     }
     if (!ring_slots<1>(need)) return SPK_OK;
     static_assert(sizeof(RedLevel) == 8 * sizeof(int), "levels are stored as eight ints");
-    SPK_TRY(s->d_red_lv.alloc(8 * (size_t)nl));
+    SPK_TRY(s->d_red_lv.reserve(8 * (size_t)nl));
     SPK_CUDA(cudaMemcpyAsync(s->d_red_lv.p, lv.data(), sizeof(RedLevel) * nl, cudaMemcpyHostToDevice, st));
     if (tot <= 2ll * span[2 * nl]) {
-        SPK_TRY(s->red_dense.alloc(tot));
+        SPK_TRY(s->red_dense.reserve(tot));
+        s->red_full = 1;
         SPK_CUDA(cudaMemsetAsync(s->red_dense.p, 0, sizeof(double) * tot, st));
         k_red_dense<<<(nk + 7) / 8, 256, 0, st>>>(nk, s->d_red_rr.p, d_level.p, s->JT.p, s->T.p,
                                                   (const RedLevel *)s->d_red_lv.p, s->red_dense.p);
@@ -606,9 +615,9 @@ int reduced_solve(spk_system *s, int fp32, int ncols, void *work, cudaStream_t s
     if (s->red_ring) {
         const int k = ring_cols(s->red_ring, ncols), slots = ring_slots(k, s->red_ring);
         int ctas = 0;
-        SPK_TRY(ring_ctas(k, fp32, !s->red_dense.p, s->red_ctas, s->red_warps, slots, &ctas));
+        SPK_TRY(ring_ctas(k, fp32, !s->red_full, s->red_ctas, s->red_warps, slots, &ctas));
         const RingLaunch R{nullptr, ring_args(s, work, slots), 1, (ncols + k - 1) / k, slots, ctas, s->red_warps, st, nullptr};
-        SPK_TRY(ring_launch(k, fp32, !s->red_dense.p, R));
+        SPK_TRY(ring_launch(k, fp32, !s->red_full, R));
     } else {
         int K = 1;
         while (K < ncols) K <<= 1;
@@ -630,7 +639,7 @@ int red_plan_build(RedPlan &p, const std::vector<RedMember> &members, int K, int
             continue;
         }
         const int k = ring_cols(m.s->red_ring, K), slots = ring_slots(k, m.s->red_ring);
-        const int w = (k == 8 ? 0 : k == 4 ? 1 : k == 2 ? 2 : 3) + (m.s->red_dense.p ? 0 : 4);
+        const int w = (k == 8 ? 0 : k == 4 ? 1 : k == 2 ? 2 : 3) + (m.s->red_full ? 0 : 4);
         ring[w].push_back(ring_args(m.s, m.work, slots));
         p.slots[w] = std::max(p.slots[w], slots);
         p.ctas[w] = std::max(p.ctas[w], m.s->red_ctas);

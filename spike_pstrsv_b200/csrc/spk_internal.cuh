@@ -84,6 +84,8 @@ struct DBuf {
         n = count;
         return SPK_OK;
     }
+    // alloc, unless what is held is large enough and at most a quarter too large
+    int reserve(size_t count) { return p && n >= count && n <= count + count / 4 ? SPK_OK : alloc(count); }
     size_t bytes() const { return n * sizeof(T); }
 };
 
@@ -197,6 +199,7 @@ struct spk_system {
     int ov_warm = 0, ov_batch_rows = 0;  // ov_batch_rows: rows per task of ov_batch, which the first batched call builds
     int batch_path = -1;      // spk_tune "batch_path": 1 chain kernels, 0 partition kernels, -1 automatic
     // 16-row records of U for the one-right-hand-side solves (sweep.cu)
+    long long sw_bytes = 0;  // of records
     int sw_ok = 0, sw_win = 0, sw_reach = 0, sw_wide = 0, sw_slots = 0, sw_stage = 0;
     spk::DBuf<unsigned char> sw_rec;
     spk::DBuf<int2> sw_hdr;
@@ -234,6 +237,7 @@ struct spk_system {
     spk::DBuf<int> d_red_lv;
     spk::DBuf<int4> d_red_rr;
     spk::DBuf<double> red_dense;
+    int red_full = 0;   // coefficients are dense (red_dense)
     int red_ring = 0;   // unknowns a level spans (0: the one-CTA solve on the CSR copy)
     int red_ctas = 1, red_warps = 8;  // CTAs per cluster, warps per CTA
     int dbg_fail_allocs = 0;  // test hook: what a batch makes on first use finds no memory, so many times (spk_debug_set)
