@@ -61,6 +61,7 @@
 #include <utility>
 #include <vector>
 
+#include "checks.cuh"
 #include "spk_internal.cuh"
 #include "sweep.cuh"
 #include "sweep_rhs.cuh"
@@ -70,23 +71,6 @@ namespace spk {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
-
-// Checked builds (-DSPK_DEVICE_CHECKS): every index of the chain kernels is
-// bounds-checked; a failed check records (code, block, index) in g_chain_check
-// (first one kept) and the access uses index 0 instead.  Off by default.
-#ifdef SPK_DEVICE_CHECKS
-__device__ unsigned long long g_chain_check;
-__device__ __noinline__ long long chk_fail(int code, long long i) {
-    atomicCAS(&g_chain_check, 0ull,
-              ((unsigned long long)code << 48) | ((unsigned long long)(blockIdx.x & 0xffffff) << 24) |
-                  (unsigned long long)(i & 0xffffff));
-    return 0;
-}
-#define CK(i, n, code) \
-    (((unsigned long long)(long long)(i) < (unsigned long long)(long long)(n)) ? (long long)(i) : chk_fail((code), (long long)(i)))
-#else
-#define CK(i, n, code) (i)
-#endif
 
 inline int nblocks(long long n, int bs = 256) { return (int)((n + bs - 1) / bs); }
 
@@ -1703,15 +1687,12 @@ int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *
     return launch_chain<true>(s, s->d_ctasks4.p + i0, i1 - i0, b, x, st);
 }
 
-// The first failed check of a checked build (0: none, or not a checked build).
+// The first failed check of a checked build in any of the solve kernels (0: none, or not a checked build).
 long long chain_device_check() {
-#ifdef SPK_DEVICE_CHECKS
-    unsigned long long v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_chain_check, sizeof(v)) != cudaSuccess) return -1;
-    return (long long)v;
-#else
+    for (long long v : {first_failed_check(), sweep_device_check(), rhs_sweep_device_check(), reduced_device_check(),
+                        residual_device_check()})
+        if (v) return v;
     return 0;
-#endif
 }
 
 // One solve through the chain path: one launch (b and x apart), or phase 1 then phase 4, on stream st.

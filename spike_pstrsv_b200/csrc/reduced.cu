@@ -12,6 +12,7 @@
 #include <map>
 #include <mutex>
 
+#include "checks.cuh"
 #include "reduced.cuh"
 
 namespace spk {
@@ -139,6 +140,8 @@ struct RingArgs {
     const int *JT;       // CSR columns
     void *xbuf;          // T, U order, leading dimension n
     int n, nred, mask;   // mask: ring slots - 1
+    int nkept;           // kept rows, coefficients, CSR entries (bounds of the checked build)
+    long long nd, nnz;
 };
 
 __device__ __forceinline__ unsigned cluster_rank() {
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
     T *xb = (T *)A.xbuf + (long long)blockIdx.y * K * A.n;
     auto fill = [&](int lo, int hi) {
         for (int id = lo + tid; id < hi; id += TH) {
-            const T *x = xb + A.mapRedX[id];
+            const T *x = xb + CK(A.mapRedX[CK(id, A.nred, 100)], A.n, 101);
 #pragma unroll
             for (int k = 0; k < K; k++) ring[(id & A.mask) * KS + k] = (double)x[(long long)k * A.n];
         }
@@ -187,24 +190,24 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
 #pragma unroll
         for (int b = 0; b < RB; b++) {
             const int q = min(gw + b, M.nr - 1);
-            rr[b] = A.rr[M.q0 + q];
+            rr[b] = A.rr[CK(M.q0 + q, A.nkept, 102)];
             if constexpr (!CSR) {
 #pragma unroll
                 for (int u = 0; u < PF; u++)
-                    pf[b][u] = lane + 32 * u < M.w ? A.D[M.d + (long long)q * M.w + lane + 32 * u] : 0.0;
+                    pf[b][u] = lane + 32 * u < M.w ? A.D[CK(M.d + (long long)q * M.w + lane + 32 * u, A.nd, 103)] : 0.0;
             }
         }
 #pragma unroll
         for (int u = 0; u < FU; u++) {
             const int id = E.f0 + tid + TH * u;
-            fid[u] = id < E.f1 ? A.mapRedX[id] : -1;
+            fid[u] = id < E.f1 ? (int)CK(A.mapRedX[CK(id, A.nred, 104)], A.n, 105) : -1;
         }
         if constexpr (CSR) {
 #pragma unroll
             for (int u = 0; u < PF; u++) {
                 const int j = rr[0].z + lane + 32 * u;
-                pf[0][u] = j < rr[0].w ? A.D[j] : 0.0;
-                pc[u] = j < rr[0].w ? A.JT[j] : 0;
+                pf[0][u] = j < rr[0].w ? A.D[CK(j, A.nd, 106)] : 0.0;
+                pc[u] = j < rr[0].w ? A.JT[CK(j, A.nnz, 107)] : 0;
             }
         }
     };
@@ -247,7 +250,7 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
             const bool first = q == gw;
             if (!first) {
 #pragma unroll
-                for (int b = 0; b < RB; b++) rr[b] = A.rr[L.q0 + min(q + b, L.nr - 1)];
+                for (int b = 0; b < RB; b++) rr[b] = A.rr[CK(L.q0 + min(q + b, L.nr - 1), A.nkept, 108)];
             }
             if constexpr (CSR) {
                 int j = rr[0].z + lane;
@@ -263,7 +266,7 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
                     double v[4];
                     int c[4];
 #pragma unroll
-                    for (int u = 0; u < 4; u++) v[u] = A.D[j + 32 * u], c[u] = A.JT[j + 32 * u];
+                    for (int u = 0; u < 4; u++) v[u] = A.D[CK(j + 32 * u, A.nd, 109)], c[u] = A.JT[CK(j + 32 * u, A.nnz, 110)];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         const double w[RB] = {v[u]};
@@ -271,13 +274,13 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
                     }
                 }
                 for (; j < je; j += 32) {
-                    const double v[RB] = {A.D[j]};
-                    step(A.JT[j], v);
+                    const double v[RB] = {A.D[CK(j, A.nd, 111)]};
+                    step(A.JT[CK(j, A.nnz, 112)], v);
                 }
             } else {
                 const double *d[RB];
 #pragma unroll
-                for (int b = 0; b < RB; b++) d[b] = A.D + L.d + (long long)min(q + b, L.nr - 1) * L.w;
+                for (int b = 0; b < RB; b++) d[b] = A.D + CK(L.d + (long long)min(q + b, L.nr - 1) * L.w, A.nd - L.w + 1, 113);
                 int c = lane;
                 if (first) {
 #pragma unroll
@@ -352,7 +355,7 @@ __global__ void __launch_bounds__(TH, TH == 256 ? 2 : 1) k_reduced_ring(const Ri
                 if (q + b < L.nr) {
                     double *slot = ring + (rr[b].x & A.mask) * KS + k;
                     const double x = *slot - acc[b][0];
-                    if (sub == 0) xb[(long long)k * A.n + rr[b].y] = (T)x;
+                    if (sub == 0) xb[(long long)k * A.n + CK(rr[b].y, A.n, 114)] = (T)x;
                     __syncwarp();  // every lane has read the old value
                     for (unsigned j = sub; j < C; j += 32 >> LK)
                         dsmem_store((unsigned)__cvta_generic_to_shared(slot), j, x);
@@ -433,7 +436,8 @@ int ring_cols(int need, int ncols) {
 RingArgs ring_args(const spk_system *s, void *work, int slots) {
     const bool dense = s->red_full;
     return RingArgs{(const RedLevel *)s->d_red_lv.p, s->nlvl, s->d_red_rr.p, s->mapRedX.p,
-                    dense ? s->red_dense.p : s->T.p, s->JT.p, work, s->n, s->nRed, slots - 1};
+                    dense ? s->red_dense.p : s->T.p, s->JT.p, work, s->n, s->nRed, slots - 1, s->nkept,
+                    (long long)(dense ? s->red_dense.n : s->T.n), (long long)s->JT.n};
 }
 
 struct RingLaunch {
@@ -536,6 +540,8 @@ RedArgs csr_args(const spk_system *s, void *work, double *red) {
 }
 
 }  // namespace
+
+long long reduced_device_check() { return first_failed_check(); }
 
 // Levels and row headers of the cluster solve from the kept rows (level by level,
 // rows/off) and each level's first reduced unknown; left unbuilt when a level

@@ -13,6 +13,7 @@
 #include <mutex>
 #include <set>
 
+#include "checks.cuh"
 #include "spk_internal.cuh"
 
 namespace spk {
@@ -39,6 +40,7 @@ struct ResArgs {
     long long ldr;
     int rev;
     unsigned long long *norms;  // max |R|, |X|, |B| per column, or null
+    long long nell;             // matrix slots (bounds of the checked build)
 };
 
 __device__ __forceinline__ void cpa(unsigned dst, const void *src, int bytes) {
@@ -54,18 +56,20 @@ __global__ void __launch_bounds__(kThreads) k_residual_block(ResArgs A) {
     int *const cs = (int *)(vs + A.slots);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * kRows;
     const int nt = (A.n + 31) >> 5, j0 = r0 >> 5, p0 = __ldg(A.ptr + j0), p1 = __ldg(A.ptr + min(j0 + kRows / 32, nt));
+    auto in_rows = [&](int c) { return (long long)r0 + CK(c - r0, A.rows, 123); };  // a column, among the rows of X copied
     auto at = [&](int r) { return A.rev ? (long long)A.n - 1 - r : (long long)r; };
     const unsigned xa = (unsigned)__cvta_generic_to_shared(xs), va = (unsigned)__cvta_generic_to_shared(vs),
                    ca = (unsigned)__cvta_generic_to_shared(cs);
     for (int e = 4 * threadIdx.x; e < p1 - p0; e += 4 * kThreads) {  // tiles hold multiples of 32 slots
-        cpa(va + 8 * e, A.ev + p0 + e, 16);
-        cpa(va + 8 * e + 16, A.ev + p0 + e + 2, 16);
-        cpa(ca + 4 * e, A.ec + p0 + e, 16);
+        const int at = (int)CK(e, A.slots - 3, 120), from = (int)CK(p0 + e, A.nell - 3, 121);
+        cpa(va + 8 * at, A.ev + from, 16);
+        cpa(va + 8 * at + 16, A.ev + from + 2, 16);
+        cpa(ca + 4 * at, A.ec + from, 16);
     }
     for (int c = warp; c < A.nk; c += W) {
         const double *x = A.X + c * A.ldx;
         for (int i = lane; i < A.rows; i += 32)
-            if (r0 + i < A.n) cpa(xa + 8 * (i * LD + c), x + at(r0 + i), 8);
+            if (r0 + i < A.n) cpa(xa + 8 * (i * LD + c), x + CK(at(r0 + i), A.n, 122), 8);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -103,8 +107,8 @@ __global__ void __launch_bounds__(kThreads) k_residual_block(ResArgs A) {
 #pragma unroll 4
             for (; k + 2 <= w; k += 2) {
                 const double v0 = ev[32 * k], v1 = ev[32 * k + 32];
-                row_of(x0 + (long long)ec[32 * k] * LD, y0);
-                row_of(x0 + (long long)ec[32 * k + 32] * LD, y1);
+                row_of(x0 + in_rows(ec[32 * k]) * LD, y0);
+                row_of(x0 + in_rows(ec[32 * k + 32]) * LD, y1);
 #pragma unroll
                 for (int u = 0; u < P; u++) {
                     a0[u] = fma(v0, y0[u], a0[u]);
@@ -113,7 +117,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_block(ResArgs A) {
             }
             if (k < w) {
                 const double v = ev[32 * k];
-                row_of(x0 + (long long)ec[32 * k] * LD, y0);
+                row_of(x0 + in_rows(ec[32 * k]) * LD, y0);
 #pragma unroll
                 for (int u = 0; u < P; u++) a0[u] = fma(v, y0[u], a0[u]);
             }
@@ -130,7 +134,7 @@ __global__ void __launch_bounds__(kThreads) k_residual_block(ResArgs A) {
                 const int c = warp + W * u;
                 if (c < A.nk) {
                     const double res = b[u] - os[lane * LD + c];
-                    A.R[c * A.ldr + o] = res;
+                    A.R[c * A.ldr + CK(o, A.n, 124)] = res;
                     mr[u] = nanmax(mr[u], fabs(res));
                     mx[u] = nanmax(mx[u], fabs(xs[(32 * t + lane) * LD + c]));
                     mb[u] = nanmax(mb[u], fabs(b[u]));
@@ -195,11 +199,14 @@ bool residual_fits(const spk_system *s, int K) {
                112 * 1024;
 }
 
+long long residual_device_check() { return first_failed_check(); }
+
 // R = B - A X (residual_fits); norms: 3 per column, zeroed before, or null.
 int residual_launch(const spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,
                     long long ldr, unsigned long long *norms, cudaStream_t st) {
     const ResArgs A{s->n, K, rows_of(s), s->ell_chunk, s->ell_ptr.p, s->ell_val.p, s->ell_col.p,
-                    s->diag.p, X, ldx, B, ldb, R, ldr, s->uplo == 'L', norms};
+                    s->diag.p, X, ldx, B, ldb, R, ldr, s->uplo == 'L', norms,
+                    (long long)s->ell_val.n};
     return K > 16 ? go<32>(A, st) : K > 8 ? go<16>(A, st) : go<8>(A, st);
 }
 

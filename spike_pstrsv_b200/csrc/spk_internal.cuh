@@ -277,6 +277,10 @@ int partition_ensure(spk_system *s);
 int chain_solve(spk_system *s, const double *b, double *x, cudaStream_t st, bool prof, int ring, bool apart);
 int chain_solve_host(spk_system *s, const double *b, double *x, double *db, double *dx);
 long long chain_device_check();
+long long sweep_device_check();
+long long rhs_sweep_device_check();
+long long reduced_device_check();
+long long residual_device_check();
 int chain_phase(spk_system *s, int phase, int row_lo, int row_hi, const double *b, double *x, cudaStream_t st);
 bool residual_fits(const spk_system *s, int K);
 int residual_launch(const spk_system *s, int K, const double *X, long long ldx, const double *B, long long ldb, double *R,

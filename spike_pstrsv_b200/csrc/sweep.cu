@@ -52,6 +52,7 @@
 #include <mutex>
 #include <set>
 
+#include "checks.cuh"
 #include "sweep.cuh"
 #include "sweep_rhs.cuh"
 
@@ -124,20 +125,20 @@ __device__ __forceinline__ bool copy_tiles(const SweepArgs &A, const Smem &M, Ri
     int2 h = make_int2(0, 0);
     for (int j = jt; j >= jb; j--) {
         const int k = (jt - j) & 31;
-        if (k == 0) h = j - lane >= jb ? __ldg(A.hdr + j - lane) : make_int2(0, 0);
+        if (k == 0) h = j - lane >= jb ? __ldg(A.hdr + CK(j - lane, (A.n + 15) >> 4, 60)) : make_int2(0, 0);
         const unsigned at = __shfl_sync(kFull, h.x, k);
-        const unsigned bytes = __shfl_sync(kFull, h.y, k);
+        const unsigned bytes = CKU(__shfl_sync(kFull, h.y, k), A.stage - 127, 61);
         const unsigned bar = M.full + 8 * R.slot, dst = M.stage0 + R.slot * A.stage;
         if (!try_wait(M.empty + 8 * R.slot, R.parity ^ 1) && !slow_wait(M.empty + 8 * R.slot, R.parity ^ 1)) return false;
         if (lane == 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                         "l"(A.rec + (unsigned long long)at * 16), "r"(bytes), "r"(bar)
+                         "l"(A.rec + CK((unsigned long long)at * 16, A.nrec - bytes + 1, 62)), "r"(bytes), "r"(bar)
                          : "memory");
         }
         const int r = 16 * j + lane;
         if (lane < 16 && r >= lo && r < hi) {
-            const double *src = A.b + (A.rev_b ? A.n - 1 - r : r);
+            const double *src = A.b + CK(A.rev_b ? A.n - 1 - r : r, A.n, 63);
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + A.stage - 128 + 8 * lane), "l"(src) : "memory");
         }
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
@@ -256,7 +257,7 @@ struct Solver {
         const unsigned gather = from, release = M.empty + 8 * R.slot, old = M.stage0 + R.slot * A.stage;
         double x[S];
 #pragma unroll
-        for (int u = 0; u < S; u++) x[u] = lds(gather + 8 * C.off(u));
+        for (int u = 0; u < S; u++) x[u] = lds(gather + 8 * CKU(C.off(u), max(A.reach, 1), 64));
         R.next(A.ns);
         if (more) {
             const unsigned bar = M.full + 8 * R.slot;
@@ -291,7 +292,7 @@ struct Solver {
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(xv) : "memory");
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + winb), "d"(xv) : "memory");
         }
-        if (row >= st_lo && row < st_hi) *xp = xv;
+        if (row >= st_lo && row < st_hi) *CKP(xp, A.x, A.n, 65) = xv;
         __syncwarp();  // the window rows; every lane is done with the stage
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(release) : "memory");
         row -= 16;
@@ -341,12 +342,12 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int r = r0 + kThreads * u + (int)threadIdx.x;
-                v[u] = r < c.y ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
+                v[u] = r < c.y ? A.pre[CK(A.rev_pre ? A.n - 1 - r : r, A.n, 66)] : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < 8; u++) {
                 const int r = r0 + kThreads * u + (int)threadIdx.x;
-                if (r < c.y) A.x[A.rev_x ? A.n - 1 - r : r] = v[u];
+                if (r < c.y) A.x[CK(A.rev_x ? A.n - 1 - r : r, A.n, 67)] = v[u];
             }
         }
         return;
@@ -390,7 +391,7 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
     auto load_window = [&](int r0, int count) {
         for (int k = lane; k < count; k += 32) {
             const int r = r0 + k;
-            const double v = A.pre && r < A.n ? A.pre[A.rev_pre ? A.n - 1 - r : r] : 0.0;
+            const double v = A.pre && r < A.n ? A.pre[CK(A.rev_pre ? A.n - 1 - r : r, A.n, 68)] : 0.0;
             const unsigned at = M.win + ((8u * (unsigned)r) & maskb);
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
             asm volatile("st.shared.f64 [%0], %1;" ::"r"(at + 8 * A.win), "d"(v) : "memory");
@@ -642,10 +643,13 @@ int sweep_prepare(spk_system *s) {
     return SPK_OK;
 }
 
+long long sweep_device_check() { return first_failed_check(); }
+
 SweepArgs sweep_args(const spk_system *s) {
     SweepArgs A{};
     A.hdr = s->sw_hdr.p;
     A.rec = s->sw_rec.p;
+    A.nrec = s->sw_bytes;
     A.n = s->n;
     A.win = s->sw_win;
     A.reach = s->sw_reach;

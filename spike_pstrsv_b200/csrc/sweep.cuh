@@ -12,6 +12,7 @@ struct SweepArgs {
     int seg;            // tasks are SegTask
     const int2 *hdr;    // per 16-row tile: record offset in 16-byte units, bytes
     const unsigned char *rec;
+    long long nrec;     // bytes of records (bounds of the checked build)
     int n;
     const double *b;    // right-hand side, caller order
     double *x;          // result

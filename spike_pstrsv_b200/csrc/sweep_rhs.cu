@@ -36,6 +36,7 @@
 
 #include <cub/cub.cuh>
 
+#include "checks.cuh"
 #include "sweep.cuh"
 #include "sweep_rhs.cuh"
 
@@ -170,7 +171,7 @@ template <typename T, int COLS, int R>
 __device__ __forceinline__ void store_tile(const RhsSweep &A, const Smem<T, COLS, R> &M, int j, int pos, int lo, int hi, int lane) {
     const int i = lane & 15, row = 16 * j + i;
     if (row < lo || row >= hi) return;
-    const long long o = A.rev_x ? (long long)A.n - 1 - row : row;
+    const long long o = CK(A.rev_x ? (long long)A.n - 1 - row : row, A.n, 84);
     const T *w = M.win + (pos + i) * M.LD;
     if (A.out_work) {
         T *x = (T *)A.X + o;
@@ -215,20 +216,20 @@ __device__ bool copy_range(const RhsSweep &A, const Smem<T, COLS, PER> &M, Ring 
         // the stage's last use: this range's, or the range's before (stored already)
         if (!(t >= A.ns ? solved() : bar_wait(M.empty + 8 * R.slot, R.parity ^ 1))) return false;
         const int j = g.jt - t, k = t & 31;
-        if (k == 0) h = j - lane >= g.jb ? __ldg(A.hdr + j - lane) : make_int2(0, 0);
-        const unsigned at = __shfl_sync(kFull, h.x, k), bytes = __shfl_sync(kFull, h.y, k);
+        if (k == 0) h = j - lane >= g.jb ? __ldg(A.hdr + CK(j - lane, (A.n + 15) >> 4, 80)) : make_int2(0, 0);
+        const unsigned at = __shfl_sync(kFull, h.x, k), bytes = CKU(__shfl_sync(kFull, h.y, k), A.stage - COLS * 17 * 8 + 1, 81);
         const unsigned bar = M.full + 8 * R.slot;
         unsigned char *dst = M.stage + (size_t)R.slot * A.stage;
         if (lane == 0) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                              su32(dst)),
-                         "l"(A.rec + (unsigned long long)at * 16), "r"(bytes), "r"(bar)
+                         "l"(A.rec + CK((unsigned long long)at * 16, A.nrec - bytes + 1, 82)), "r"(bytes), "r"(bar)
                          : "memory");
         }
         const int i = lane & 15, row = 16 * j + i;
         if (row >= g.lo && row < g.hi) {
-            const double *src = A.B + (A.rev_b ? (long long)A.n - 1 - row : (long long)row);
+            const double *src = A.B + CK(A.rev_b ? (long long)A.n - 1 - row : (long long)row, A.n, 83);
             const unsigned b = su32(dst + A.stage - COLS * 17 * 8) + 8 * i;
 #pragma unroll 4
             for (int c = lane >> 4; c < A.nk; c += 2)
@@ -289,10 +290,10 @@ __device__ bool solve_range(const RhsSweep &A, const Smem<T, NW * 8 * R, R> &M, 
             const unsigned from = has >> 4 * k & 1 ? gat : zero;  // distances of a row without any are 0
 #pragma unroll
             for (int e = 0; e < C; e++) {
-                lds(from + o[e].x * LD, x[4 * e]);
-                lds(from + o[e].y * LD, x[4 * e + 1]);
-                lds(from + o[e].z * LD, x[4 * e + 2]);
-                lds(from + o[e].w * LD, x[4 * e + 3]);
+                lds(from + CKU(o[e].x, max(A.reach, 1), 85) * LD, x[4 * e]);
+                lds(from + CKU(o[e].y, max(A.reach, 1), 85) * LD, x[4 * e + 1]);
+                lds(from + CKU(o[e].z, max(A.reach, 1), 85) * LD, x[4 * e + 2]);
+                lds(from + CKU(o[e].w, max(A.reach, 1), 85) * LD, x[4 * e + 3]);
             }
             lds(val + 4 * C * B * (4 * k + q), v);
             if (k < 3)
@@ -338,8 +339,8 @@ __device__ bool solve_range(const RhsSweep &A, const Smem<T, NW * 8 * R, R> &M, 
                 const int4 at = ldsi4(ex + 16 * e);
                 if ((at.x & 3) == q && !(top && 16 * j + at.x >= g.hi) && !(bottom && 16 * j + at.x < g.lo)) {
                     T x[R], y[R];
-                    lds(gat + at.y * LD, x);
-                    lds(rcol + at.x * LD, y);
+                    lds(gat + CKU(at.y, max(A.reach, 1), 86) * LD, x);
+                    lds(rcol + CKU(at.x, 16, 87) * LD, y);
                     const T v = (T)__hiloint2double(at.w, at.z);
 #pragma unroll
                     for (int u = 0; u < R; u++) y[u] = fma(-v, x[u], y[u]);
@@ -397,7 +398,7 @@ __device__ __forceinline__ void rhs_task(const RhsSweep &A, int task) {
         const T *pre = (const T *)A.pre;
         for (int k = 0; k < A.nk; k++)
             for (int r = c.x + (int)threadIdx.x; r < c.y; r += blockDim.x) {
-                double *x = (double *)A.X + k * A.ldx + (A.rev_x ? A.n - 1 - r : r);
+                double *x = (double *)A.X + k * A.ldx + CK(A.rev_x ? A.n - 1 - r : r, A.n, 88);
                 const double v = (double)pre[(long long)k * A.n + r];
                 *x = A.acc ? *x + v : v;
             }
@@ -431,7 +432,7 @@ __device__ __forceinline__ void rhs_task(const RhsSweep &A, int task) {
         for (int e = threadIdx.x; e < count * COLS; e += NW * 32) {
             const int k = e / count, i = e - k * count, r = r0 + i, p = p0 + i >= A.win ? p0 + i - A.win : p0 + i;
             const T v = pre && r < A.n && k < A.nk ? pre[(long long)k * A.n + r] : T(0);
-            M.win[p * LD + k] = v;
+            M.win[CK(p, A.win, 89) * LD + k] = v;
             if (p < A.mirror) M.win[(p + A.win) * LD + k] = v;
         }
     };
@@ -731,10 +732,13 @@ int rhs_sweep_prepare(spk_system *s, int fp32) {
     return SPK_OK;
 }
 
+long long rhs_sweep_device_check() { return first_failed_check(); }
+
 RhsSweep rhs_sweep_args(const spk_system *s, int fp32, int nk) {
     RhsSweep A{};
     A.hdr = s->rs_hdr[fp32].p;
     A.rec = s->rs_rec[fp32].p;
+    A.nrec = (long long)s->rs_rec[fp32].n;
     A.n = s->n;
     A.nk = nk;
     A.reach = s->sw_reach;

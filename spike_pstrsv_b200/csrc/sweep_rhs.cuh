@@ -10,6 +10,7 @@ struct RhsSweep {
     int ntasks, seg;
     const int2 *hdr;    // per 16-row tile: record offset in 16-byte units, bytes
     const unsigned char *rec;
+    long long nrec;     // bytes of records (bounds of the checked build)
     int n, nk;          // rows; right-hand sides of this pass
     const double *B;    // caller order, column-major
     long long ldb;
