@@ -204,7 +204,8 @@ struct spk_system {
     spk::DBuf<unsigned char> sw_rec;
     spk::DBuf<int2> sw_hdr;
     // the same for many right-hand sides (sweep_rhs.cu; [0] FP64, [1] FP32; made on first use)
-    int rs_ok[2] = {0, 0}, rs_bytes[2] = {0, 0}, rs_groups = 0, rs_extras = 0;
+    int rs_ok[2] = {0, 0}, rs_bytes[2] = {0, 0}, rs_groups = 0;
+    long long rs_extras = 0;  // coefficients past the common ones
     spk::DBuf<unsigned char> rs_rec[2];
     spk::DBuf<int2> rs_hdr[2];
     spk::DBuf<int2> d_copies;  // phase 3+4: row ranges that keep their phase-1 values

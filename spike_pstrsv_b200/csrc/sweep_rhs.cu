@@ -682,10 +682,10 @@ void rhs_sweep_choose(spk_system *s, const int *hist, int most) {
     s->rs_groups = 0;
     for (int c : kGroups) {
         double cost = 0;
-        int extras = 0;
+        long long extras = 0;
         for (int k = 0; k <= most; k++) {
             cost += hist[k] * (4.0 * c + 60.0 * std::max(0, k - 4 * c));
-            if (hist[k] && k > 4 * c) extras = 1;
+            extras += (long long)hist[k] * std::max(0, k - 4 * c);
         }
         if (!s->rs_groups || cost < best) s->rs_groups = c, s->rs_extras = extras, best = cost;
     }
@@ -697,7 +697,7 @@ int rhs_sweep_prepare(spk_system *s, int fp32) {
     const int nt = (s->n + 15) / 16, S = s->sw_slots, C = s->rs_groups, blocks = (nt + 3) / 4;
     const int base = fp32 ? base_bytes<float>(C) : base_bytes<double>(C);
     cudaStream_t st = s->stream;
-    if ((long long)nt * (base / 16 + 16 * 128) >= (1ll << 32)) return SPK_OK;  // offsets are 32-bit
+    if ((long long)nt * (base / 16) + s->rs_extras >= (1ll << 32)) return SPK_OK;  // offsets are 32-bit, in 16 bytes
     SPK_TRY(s->rs_hdr[fp32].alloc(nt));
     unsigned all = (unsigned)nt * (base / 16), most = base / 16;
     if (s->rs_extras) {
@@ -721,7 +721,7 @@ int rhs_sweep_prepare(spk_system *s, int fp32) {
     }
     SPK_TRY(s->rs_rec[fp32].alloc((size_t)all * 16));
     auto fill = [&](auto kern) {
-        kern<<<blocks, 128, 0, st>>>(nt, s->sw_hdr.p, s->sw_rec.p, S, C, s->rs_extras, s->rs_hdr[fp32].p, s->rs_rec[fp32].p);
+        kern<<<blocks, 128, 0, st>>>(nt, s->sw_hdr.p, s->sw_rec.p, S, C, s->rs_extras > 0, s->rs_hdr[fp32].p, s->rs_rec[fp32].p);
     };
     if (fp32) s->sw_wide ? fill(k_rhs_fill<float, true>) : fill(k_rhs_fill<float, false>);
     else s->sw_wide ? fill(k_rhs_fill<double, true>) : fill(k_rhs_fill<double, false>);
