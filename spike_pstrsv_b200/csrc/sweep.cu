@@ -53,6 +53,7 @@
 #include <set>
 
 #include "checks.cuh"
+#include "records.cuh"
 #include "sweep.cuh"
 #include "sweep_rhs.cuh"
 
@@ -60,42 +61,15 @@ namespace spk {
 
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 64;        // a solving and a copying warp
 constexpr int kMaxSlots = 64;       // slots per lane
 constexpr int kMaxWindow = 8192;    // rows
 constexpr double kGrowth = 4.0;     // largest absolute row sum of W
-// record: W, 1 / diagonal, then the number of extra slots (low 16 bits) and the rows that have a
-// column outside the tile (a bit each above them), the slots' values and offsets, the extra slots'
-constexpr int kExtra = 1024 + 128;
-constexpr int kHead = kExtra + 16;
-constexpr long long kWaitCycles = 1ll << 32;  // ~2 s: bound of a barrier wait
 constexpr int kCopyRows = 1024;     // rows per copy block
 constexpr int kMaxStages = 9;
 
 constexpr int kSlots[] = {2, 4, 6, 8, 10, 12, 16, 20};  // slots per lane on the common path
 
-// Bytes of S slots per lane: values, and offsets in words (S even; four or two a word).
-__host__ __device__ constexpr int slot_bytes(int S, bool wide) { return 256 * S + 128 * (wide ? S / 2 : (S + 3) / 4); }
-
-__device__ __forceinline__ unsigned su32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool try_wait(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __noinline__ bool slow_wait(unsigned bar, unsigned parity) {
-    const long long t0 = clock64();
-    while (!try_wait(bar, parity))
-        if (clock64() - t0 > kWaitCycles) return false;
-    return true;
-}
 __device__ __forceinline__ double lds(unsigned a) {
     double v;
     asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
@@ -107,16 +81,6 @@ struct Smem {
     unsigned full, empty, zero, win, stage0;
     __device__ explicit Smem(unsigned base, int win_rows)
         : full(base), empty(base + 8 * kMaxStages), zero(base + 16 * kMaxStages), win(base + 256), stage0(base + 256 + 16 * win_rows) {}
-};
-
-struct Ring {  // the stage a warp is at, and the parity of its next completion
-    int slot = 0, parity = 0;
-    __device__ void next(int ns) {
-        if (++slot == ns) {
-            slot = 0;
-            parity ^= 1;
-        }
-    }
 };
 
 // The copying warp: tiles of rows [lo, hi), top first.
@@ -169,7 +133,7 @@ struct Record {
 #pragma unroll
         for (int h = 0; h < S / 2; h++) lds2(st + kHead + 512 * h + 16 * lane, v[2 * h], v[2 * h + 1]);
         b = lds(st + boff + 8 * myrow);
-        rd = lds(st + 1024 + 8 * myrow);
+        rd = lds(st + kDiag + 8 * myrow);
 #pragma unroll
         for (int h = 0; h < 2; h++) lds2(st + 512 * h + 16 * lane, w[2 * h], w[2 * h + 1]);
     }
@@ -484,7 +448,7 @@ __global__ void __launch_bounds__(128) k_sweep_fill(int n, int ntiles, const int
         rd = 1.0 / a[b];
     }
     if (lane < 16) {
-        ((double *)(R + 1024))[i] = rd;
+        ((double *)(R + kDiag))[i] = rd;
         for (int q = b + 1; q < f; q++) t[i][ja[q] - row0] = a[q] * rd;
     }
     __syncwarp();
@@ -531,24 +495,6 @@ __global__ void __launch_bounds__(128) k_sweep_fill(int n, int ntiles, const int
     };
     put(R + kHead, S0, 0);
     if (E) put(R + kHead + slot_bytes(S0, WIDE), E, S0);
-}
-
-// The dynamic shared memory of a kernel, raised once per device to the opt-in maximum
-// (launches come from several host threads).
-template <typename K>
-int allow_smem(K kern) {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> done;
-    int dev = 0;
-    SPK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
-    const auto key = std::make_pair(dev, (const void *)kern);
-    if (done.count(key)) return SPK_OK;
-    int mx = 0;
-    SPK_CUDA(cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    done.insert(key);
-    return SPK_OK;
 }
 
 }  // namespace

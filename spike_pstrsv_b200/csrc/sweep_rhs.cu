@@ -37,6 +37,7 @@
 #include <cub/cub.cuh>
 
 #include "checks.cuh"
+#include "records.cuh"
 #include "sweep.cuh"
 #include "sweep_rhs.cuh"
 
@@ -44,8 +45,6 @@ namespace spk {
 
 namespace {
 
-constexpr unsigned kFull = 0xffffffffu;
-constexpr long long kWaitCycles = 1ll << 32;  // ~2 s: bound of a barrier wait
 constexpr int kMaxStages = 4;
 constexpr size_t kMaxSmem = 220 * 1024;
 constexpr int kGroups[] = {1, 2, 3, 4, 5, 6};  // C: groups of four outside coefficients a row
@@ -62,24 +61,6 @@ __host__ __device__ constexpr int base_bytes(int C) { return head_bytes<T>() + 6
 // and the rows that have a column outside the tile (a bit each; the others read a zero row beside
 // the window, not one they do not depend on); then the extras, 16 bytes each: row, distance, value (FP64)
 
-__device__ __forceinline__ unsigned su32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool try_wait(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __noinline__ bool slow_wait(unsigned bar, unsigned parity) {
-    const long long t0 = clock64();
-    while (!try_wait(bar, parity))
-        if (clock64() - t0 > kWaitCycles) return false;
-    return true;
-}
 __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) { return try_wait(bar, parity) || slow_wait(bar, parity); }
 
 // N consecutive values in shared memory (32-bit addresses), in the widest pieces that the
@@ -130,16 +111,6 @@ __device__ __forceinline__ void sts(unsigned a, const float (&v)[N]) {
     if constexpr (N == 1) asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v[0]) : "memory");
     else asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v[0]), "f"(v[1]) : "memory");
 }
-
-struct Ring {
-    int slot = 0, parity = 0;
-    __device__ void next(int ns) {
-        if (++slot == ns) {
-            slot = 0;
-            parity ^= 1;
-        }
-    }
-};
 
 // Shared memory of a task: barriers, r of the tile, a zero row, the window (win + mirror rows), the stages.
 // COLS columns padded to keep rows aligned for reads of R columns.
@@ -477,11 +448,10 @@ __global__ void __launch_bounds__(32 * (NW + 1)) k_sweep_rhs(const RhsSweep *__r
 // A lane's slots in the one-right-hand-side record: slot u of S (then of the E extra).
 template <bool WIDE>
 __device__ __forceinline__ void sw_slot(const unsigned char *R, int S, int E, int u, int lane, double &v, int &o) {
-    // (sweep.cu: W 1024 bytes, 1 / diagonal 128, number of extra slots 16, then values and offsets)
-    const unsigned char *at = R + 1168;
+    const unsigned char *at = R + kHead;
     int count = S;
     if (u >= S) {
-        at += 256 * S + 128 * (WIDE ? S / 2 : (S + 3) / 4);
+        at += slot_bytes(S, WIDE);
         count = E;
         u -= S;
     }
@@ -490,7 +460,7 @@ __device__ __forceinline__ void sw_slot(const unsigned char *R, int S, int E, in
     o = WIDE ? ((const unsigned short *)at)[((u >> 1) * 32 + lane) * 2 + (u & 1)] : at[((u >> 2) * 32 + lane) * 4 + (u & 3)];
 }
 
-__device__ __forceinline__ int extra_slots(const unsigned char *R) { return *(const int *)(R + 1152) & 0xffff; }
+__device__ __forceinline__ int extra_slots(const unsigned char *R) { return *(const int *)(R + kExtra) & 0xffff; }
 
 __device__ __forceinline__ int lane_row(int lane) { return (lane & 2) ? 15 - (lane >> 2) : lane >> 2; }
 
@@ -552,7 +522,7 @@ __global__ void k_rhs_fill(int nt, const int2 *__restrict__ sw_hdr, const unsign
         }
         W[at] = (T)v;
     }
-    if (lane < 16) ((double *)(W + 160))[lane] = ((const double *)(R + 1024))[lane];
+    if (lane < 16) ((double *)(W + 160))[lane] = ((const double *)(R + kDiag))[lane];
     // extras of the rows before each: rows in order
     const int mine = lane & 15, held = row_count<WIDE>(R, S, E, lane);
     const int c = __shfl_sync(kFull, held, mine < 8 ? 4 * mine : 4 * (15 - mine) + 2), ex = max(0, c - 4 * C);
@@ -593,22 +563,6 @@ __global__ void k_rhs_fill(int nt, const int2 *__restrict__ sw_hdr, const unsign
 
 // ---- host ---------------------------------------------------------------------------
 
-template <typename K>
-int allow_smem(K kern) {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> done;
-    int dev = 0;
-    SPK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
-    const auto key = std::make_pair(dev, (const void *)kern);
-    if (done.count(key)) return SPK_OK;
-    int mx = 0;
-    SPK_CUDA(cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    done.insert(key);
-    return SPK_OK;
-}
-
 struct Launch {
     const RhsSweep *tab;
     const int2 *work;
@@ -616,17 +570,12 @@ struct Launch {
     int blocks;
     size_t smem;
     cudaStream_t st;
-    int *occ;  // query instead of launch
 };
 
 template <typename T, int PER, int NW, int C>
 int launch_one(const Launch &L) {
     auto kern = k_sweep_rhs<T, PER, NW, C>;
     SPK_TRY(allow_smem(kern));
-    if (L.occ) {
-        SPK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(L.occ, kern, 32 * (NW + 1), L.smem));
-        return SPK_OK;
-    }
     kern<<<L.blocks, 32 * (NW + 1), L.smem, L.st>>>(L.tab, L.work, L.one);
     SPK_CUDA(cudaGetLastError());
     return SPK_OK;
@@ -769,13 +718,6 @@ bool rhs_sweep_fits(const spk_system *s, int fp32, int nk) {
 
 int rhs_sweep_class(const spk_system *s, int fp32, int nk) {
     return 16 * rhs_sweep_args(s, fp32, nk).shape + s->rs_groups;
-}
-
-int rhs_sweep_occupancy(const spk_system *s, int fp32, int nk, int *occ) {
-    Launch L{};
-    L.smem = rhs_sweep_smem(s, fp32, nk);
-    L.occ = occ;
-    return launch_class(rhs_sweep_class(s, fp32, nk), fp32, L);
 }
 
 int rhs_sweep_launch(const spk_system *s, const RhsSweep &A, int fp32, cudaStream_t st) {

@@ -41,7 +41,6 @@ void rhs_sweep_release(spk_system *s);
 // Whether nk right-hand sides fit (the window of wide rows may not).
 bool rhs_sweep_fits(const spk_system *s, int fp32, int nk);
 RhsSweep rhs_sweep_args(const spk_system *s, int fp32, int nk);
-int rhs_sweep_occupancy(const spk_system *s, int fp32, int nk, int *occ);
 int rhs_sweep_launch(const spk_system *s, const RhsSweep &A, int fp32, cudaStream_t st);
 // Shared memory and kernel class of a launch; launches of one class may be joined.
 int rhs_sweep_class(const spk_system *s, int fp32, int nk);
