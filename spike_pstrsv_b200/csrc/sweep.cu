@@ -342,11 +342,12 @@ __device__ __forceinline__ void sweep_task(const SweepArgs &A, int task) {
         bool ok = true;
         if (first) ok = copy_tiles(A, M, R, lo1, hi, lane);
         if (then && ok) ok = copy_tiles(A, M, R, lo, skip_lo, lane);
-        // no copy may land after the block is gone: the stages still in flight
+        // no copy may land after the block is gone: the stages still in flight (a stage not filled
+        // yet is asked for the parity before its first, which a new barrier has)
         for (int k = 0; k < A.ns; k++) {
             if (R.slot == 0) R.parity ^= 1;
             R.slot = R.slot == 0 ? A.ns - 1 : R.slot - 1;
-            if (k < (hi - lo + 15) / 16) slow_wait(M.full + 8 * R.slot, R.parity);
+            slow_wait(M.full + 8 * R.slot, R.parity);
         }
         return;
     }
