@@ -153,7 +153,7 @@ int spk_solve(spk_system *s, const double *b, double *x);
 /* Batched solve of nrhs right-hand sides, device arrays, column-major (column k
  * of B at B + k*ldb, of X at X + k*ldx), asynchronous on `stream` unless a
  * residual is requested or tol >= 0.  The matrix is read once per group of up
- * to 16 right-hand sides.
+ * to 32 right-hand sides (16 where a system has no 16-row records).
  *   mode SPK_MODE_FP64:    FP64 tile solves.
  *   mode SPK_MODE_FP32_IR: FP32 tile solves (FP32 values, FP32 accumulation), FP64
  *     residual R = B - A X and FP64 update X += solve_fp32(R), repeated until the

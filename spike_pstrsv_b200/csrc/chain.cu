@@ -32,7 +32,7 @@
 // is free, down to 32 rows, and the walk's length is a + ov_warm instead of at least
 // twice the decay length.  They read b of rows that other tasks store: an x in b's place
 // takes the two phases, whose tasks read b of their own rows only (phase 4 of rows that
-// phase 1 has not stored).  262,147 rows, transpose: 80 -> 48 us; 5,003 rows: 47 -> 27 us.
+// phase 1 has not stored).  262,147 rows, transpose: 80 -> 49 us; 5,003 rows: 47 -> 24 us.
 // spk_chain_phase keeps the two phases (a shard's rows end where another GPU's start).
 //
 // Kernel (systems without records, and the phases' layout).  One warp per task, lane = row of
@@ -1246,8 +1246,10 @@ int batch_chains(spk_system *s) {
 // Rows per task of the batched one-launch solve: two tasks an SM once a task's own rows
 // outnumber the rows it walks before them, else one (two slow each other down by 1.1, with
 // 17 and more right-hand sides by 1.6).  FP64, one / two / three tasks: 32 right-hand sides,
-// 4,194,304 banded rows 1,767 / 1,446 / 1,630 us, 20,011 rows 127 / 185 / 210 us; 300,007 rows,
-// 21: 220 / 248 / 424 us, 12: 207 / 160 / 186 us, 4: 187 / 143 / 163 us.
+// 4,194,304 banded rows 1,735 / 1,430 / 1,607 us (16: 1,506 / 855 / 826), 20,011 rows 78 / 113 / 172
+// us; 300,007 rows, 21: 213 / 244 / 420 us, 12: 197 / 152 / 183 us, 4: 181 / 139 / 159 us.  A system
+// has one plan whatever the number of columns, so between the two (300,007 rows) it is the one
+// for few columns, and 17 and more take a seventh longer than they could.
 long long batch_overlap_rows(const spk_system *s, int sms) {
     if (const char *e = getenv("SPK_CHAIN_BATCH_ROWS")) return std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     const long long w = s->n / sms >= overlap_warm(s) ? 2 : 1;
@@ -1256,11 +1258,13 @@ long long batch_overlap_rows(const spk_system *s, int sms) {
 
 // Rows per task of the one-launch solve.  With w tasks an SM a task walks n / (sms w) +
 // ov_warm rows: more tasks shorten the walk, but slow each other down and together
-// walk more rows, until the records saturate HBM.  Measured, w = 1 .. 6: 262,147 banded
-// rows 78 / 57 / 57 / 53 / 55 / 55 us, 4,194,304 rows 706 / 371 / 295 / 232 / 213 / 189 us (the
-// transpose, with longer records, 235 us from w = 4 on), 65,536 rows 46 / 41 / 44 / 43 / 47 us;
-// the model is within 6 % of those: 0.27 us and 0.012 us a slot per tile, 6 % more for
-// each further task, 6.5 TB/s.
+// walk more rows, until the records saturate HBM.  Measured back to back, w = 1 .. 6: 65,536
+// banded rows 41 / 35 / 37 / 37 / 40 / 40 us, 262,147 rows 72 / 51 / 49 / 45 / 49 / 47 us (the
+// transpose 74 / 54 / 51 / 48 / 52 / 51), 4,194,304 rows 712 / 374 / 293 / 229 / 216 / 191 us (the
+// transpose, with longer records, 708 / 375 / 293 / 239 / 236; six do not fit an SM).  The model
+// (0.27 us and 0.012 us a slot per tile, 6 % more for each further task, 6.5 TB/s) is up to 11 %
+// below those at full size and up to 20 % below at the small ones, where it leaves the launch
+// out; it takes the fastest w of each line.
 long long overlap_rows(spk_system *s, int sms, int occ) {
     if (const char *e = getenv("SPK_CHAIN_ROWS")) return std::max(32ll, 32ll * ((atoll(e) + 31) / 32));
     const long long n = s->n, warm = overlap_warm(s);

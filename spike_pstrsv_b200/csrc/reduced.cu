@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(red_threads<K>()) k_reduced_csr(const RedArgs 
 // so that an unknown reaches the rows that read it and no others.  Otherwise they stay in CSR order.
 //
 // Measured (one right-hand side, this kernel alone against one CTA on the CSR
-// copy): banded rows, 524,288 rows in 128 partitions, 126 levels of 61 rows: 690 ->
+// copy; the look at every row's sum has since added 1 to 2 %): banded rows, 524,288 rows in 128 partitions, 126 levels of 61 rows: 690 ->
 // 218 us (1.7 us a level: the barrier's release waits 0.4 us for the remote stores, the rest
 // is one row's dependent steps; loading all of it two levels ahead changed nothing);
 // band of 200, 100,003 rows in 48 partitions, 46 levels of 176 rows: 958 -> 90 us (170 with

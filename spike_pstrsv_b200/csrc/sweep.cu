@@ -34,12 +34,13 @@
 //   choice is made on the address, a tile ahead: it costs nothing there (128 x 128 Poisson factor
 //   160 us, 176 us where the sum was dropped instead, on the way from one tile to the next).
 //
-// Measured (one solve, before -> after): banded rows with 16 off-diagonals, 4,194,304
-// rows: lower 234 -> 206 us (6 tasks an SM, 233 bytes a row: bound by HBM), its transpose
-// 573 -> 246 us; 262,147 rows, transpose: 264 -> 80 us (0.40 us a tile of 16 rows: its
-// latency); 128 x 128 Poisson factor in 4 partitions: 298 -> 160 us (0.28 us a tile).
-// Staged records: 2 / 3 / 4 / 6 a task take 180 / 99 / 80 / 80 us at 262,147 rows and 3 / 4 /
-// 5 / 6 take 233 / 211 / 208 / 194 us at full size.
+// Measured (one solve, the row-by-row kernels -> this one): banded rows with 16 off-diagonals,
+// 4,194,304 rows: lower 234 -> 201 to 212 us (191 back to back; 6 tasks an SM, 233 bytes a row:
+// bound by HBM), its transpose 573 -> 250 us; 262,147 rows, transpose, in the same two phases: 264
+// -> 80 us (0.40 us a tile of 16 rows: its latency), in the one launch that plain solves take 50 us
+// (chain.cu); 128 x 128 Poisson factor in 4 partitions: 298 -> 160 us (0.28 us a tile).
+// Staged records (two phases): 2 / 3 / 4 / 6 a task take 180 / 99 / 80 / 80 us at 262,147 rows and
+// 3 / 4 / 5 / 6 take 233 / 211 / 208 / 194 us at full size.
 //
 // W is used only where its rows' absolute sums stay at most kGrowth: the error of the product
 // grows with them (c u |W||T||W||r| against c u |W||T||x| of the substitution).  Over 40,000 random
