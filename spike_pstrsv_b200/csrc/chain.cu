@@ -55,8 +55,6 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
-#include <mutex>
-#include <set>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -73,27 +71,6 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 
 inline int nblocks(long long n, int bs = 256) { return (int)((n + bs - 1) / bs); }
-
-// The dynamic shared memory a kernel may take, raised once per kernel and device
-// to the device's opt-in maximum.  Launches of the same kernel for systems of
-// different sizes come from several host threads (the serving loop's workers);
-// setting the attribute to each launch's own size would race with the launches
-// of other threads.
-template <typename K>
-int allow_smem(K kern) {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> done;
-    int dev = 0;
-    SPK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
-    const auto key = std::make_pair(dev, (const void *)kern);
-    if (done.count(key)) return SPK_OK;
-    int mx = 0;
-    SPK_CUDA(cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    done.insert(key);
-    return SPK_OK;
-}
 
 // ---- layout construction -----------------------------------------------------------
 

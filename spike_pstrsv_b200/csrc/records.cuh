@@ -2,10 +2,6 @@
 // (sweep_rhs.cu) are made from, and what both kernels share: the ring of stages and its waits.
 #pragma once
 
-#include <mutex>
-#include <set>
-#include <utility>
-
 #include "spk_internal.cuh"
 
 namespace spk {
@@ -51,24 +47,6 @@ struct Ring {  // the stage a warp is at, and the parity of its next completion
         }
     }
 };
-
-// The dynamic shared memory of a kernel, raised once per device to the opt-in maximum
-// (launches come from several host threads).
-template <typename K>
-int allow_smem(K kern) {
-    static std::mutex mu;
-    static std::set<std::pair<int, const void *>> done;
-    int dev = 0;
-    SPK_CUDA(cudaGetDevice(&dev));
-    std::lock_guard<std::mutex> g(mu);
-    const auto key = std::make_pair(dev, (const void *)kern);
-    if (done.count(key)) return SPK_OK;
-    int mx = 0;
-    SPK_CUDA(cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    done.insert(key);
-    return SPK_OK;
-}
 
 }  // namespace
 }  // namespace spk

@@ -14,7 +14,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/spike_pstrsv.h"
@@ -298,6 +301,27 @@ int collect_event_set(spk_system *s, int k);
 // of the one-launch solves read rows of b that other tasks store x of, so they need it; the two
 // phases and the partitions read a task's own rows only, before they are stored.
 bool columns_apart(long long n, int nrhs, const double *B, long long ldb, const double *X, long long ldx);
+
+// The dynamic shared memory a kernel may take, raised once per kernel and device
+// to the device's opt-in maximum.  Launches of the same kernel for systems of
+// different sizes come from several host threads (the serving loop's workers);
+// setting the attribute to each launch's own size would race with the launches
+// of other threads.
+template <typename K>
+int allow_smem(K kern) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void *>> done;
+    int dev = 0;
+    SPK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(mu);
+    const auto key = std::make_pair(dev, (const void *)kern);
+    if (done.count(key)) return SPK_OK;
+    int mx = 0;
+    SPK_CUDA(cudaDeviceGetAttribute(&mx, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    SPK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    done.insert(key);
+    return SPK_OK;
+}
 
 // pointer classification
 int is_device_pointer(const void *p);
