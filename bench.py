@@ -486,7 +486,7 @@ def run_ours(args):
     achieved = B / (kernel_ms * 1e-3) / 1e9
     kernel_rows_gbs = (B / m) * (rows1 + rows4) / (kernel_ms * 1e-3) / 1e9
     traffic = None
-    tp = os.path.join(ROOT, "profiles", "chain_solve_traffic.json" if chain else "tile_solve_traffic.json")
+    tp = os.path.join(ROOT, "profiles", "sweep_traffic.json" if chain else "tile_solve_traffic.json")
     if os.path.exists(tp):
         with open(tp) as f:
             tr = json.load(f)
